@@ -1,0 +1,80 @@
+"""The solver of models of several kinematic trees (nv > 32) over nonzero trees and tiles only, at the
+edges of its structure: 2 to 65 trees (64 is the most that it takes), tree sizes 6 and 27, matrices
+whose last 32-dof panel is partial, worlds without rows, rows past its row capacity."""
+
+import numpy as np
+import pytest
+import torch
+
+import mjx_warp_b200 as mjw
+from mjx_warp_b200.types import MJ_JAC_DENSE
+from helpers import dev, device_data, load, world_rows
+from test_gpu_configs import bin_state, humanoid_spheres_state
+
+pytestmark = pytest.mark.gpu
+
+
+def spheres_xml(n):
+  """n free spheres on a grid over a plane, every other one touching it."""
+  bodies = "\n".join(
+    f'<body pos="{0.3 * (i % 9):.2f} {0.3 * (i // 9):.2f} {0.095 if i % 2 else 0.5}"><freejoint/>'
+    f'<geom type="sphere" size="0.1"/></body>' for i in range(n))
+  return ('<mujoco><option timestep="0.002"/><worldbody><geom type="plane" size="0 0 1"/>'
+          + bodies + "</worldbody></mujoco>")
+
+
+def case(name):
+  """(model, qpos, qvel, ctrl, rows capacity per world)"""
+  opt = dict(iterations=0, ls_iterations=10, jacobian=MJ_JAC_DENSE)
+  if name.startswith("spheres"):
+    mjm = load(spheres_xml(int(name[7:])), **opt)
+    rng = np.random.default_rng(1)
+    q = np.tile(mjm.qpos0, (5, 1))
+    x = q.reshape(5, -1, 7)
+    x[:, :, :2] += rng.uniform(-0.12, 0.12, x[:, :, :2].shape)
+    x[0, :, 2] += 5.0  # a world without rows
+    return mjm, q, rng.normal(0.0, 0.1, (5, mjm.nv)), np.zeros((5, 0)), 512
+  if name == "humanoid_spheres":
+    mjm = load("humanoid_spheres.xml", **opt)
+    q, v, u, _ = humanoid_spheres_state(mjm, load("humanoid.xml"), 8, seed=3)
+    return mjm, q, v, u, 384
+  mjm = load("bin.xml", **opt)
+  q, v, u = bin_state(mjm, 4, seed=6)
+  if name == "bin_rows":  # every body in one heap in worlds 0 and 1
+    x = q.reshape(4, -1, 7)
+    x[:2, :, :3] = np.array([0.0, 0.0, 0.3]) + 0.28 * (x[:2, :, :3] - np.array([0.0, 0.0, 0.19]))
+  return mjm, q, v, u, 2048
+
+
+@pytest.mark.parametrize("warps", [2, 4])
+@pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres64", "spheres65", "humanoid_spheres",
+                                  "bin", "bin_rows"])
+def test_factor_of_the_hessian(name, warps):
+  """With no iterations efc_h is the factor of H = qM + J_a' D_a J_a at the warmstart's active set:
+  zero where H's factor is, and L L' = H within the backward error of an FP32 Cholesky factorisation
+  (nv + 1 roundings of 2^-24 per entry, doubled for the assembly)."""
+  mjm, q, v, u, cap = case(name)
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, u, nconmax=800 * nworld, njmax=cap * nworld)
+  try:
+    mjw.set_tune(m, d, solver_cta_warps=warps)
+    mjw.forward(m, d)
+    torch.cuda.synchronize()
+  finally:
+    mjw.set_tune(m, d, solver_cta_warps=4 if mjm.nv > 128 else 0)
+  assert np.all(mjw.world_status(d) == 0)
+  n, idx = world_rows(d, "efc")
+  if name == "bin_rows":
+    assert n.max() > 736 > n.min()
+  J, D = (x.cpu().numpy().astype(np.float64) for x in (d.efc.J, d.efc.D))
+  act = d.efc.active.cpu().numpy().astype(bool)
+  at = 0
+  for w in range(nworld):
+    rows = idx[at:at + n[w]]
+    at += n[w]
+    rows = rows[act[rows]]
+    H = d.qM[w].cpu().numpy().astype(np.float64) + J[rows].T @ (D[rows, None] * J[rows])
+    L = np.tril(d.efc.h[w].cpu().numpy().astype(np.float64))
+    r = np.linalg.norm(L @ L.T - H) / np.linalg.norm(H)
+    assert r < 2 * (mjm.nv + 1) * 2.0 ** -24, (w, r)
