@@ -205,12 +205,15 @@ __device__ __forceinline__ bool in_bracket(const float* x, const float* y) {
   return (x[1] < y[1] && y[1] < 0.f) || (x[1] > y[1] && y[1] > 0.f);
 }
 
-// solver.py:737-869 with the iterative (:339-664) or parallel (:667-734) line search
-__device__ void linesearch(SolverCtx& s) {
+// solver.py:737-869 with the iterative (:339-664) or parallel (:667-734) line search.  mulm() forms
+// s.mv = M s.search, rowdot(k) gives row k's J . s.search, evalg evaluates the smooth part's
+// polynomial (eval_pt3).
+template <class MulM, class RowDot, class EvalG>
+__device__ __forceinline__ void linesearch_with(SolverCtx& s, MulM&& mulm, RowDot&& rowdot, EvalG&& evalg) {
   const MjbModel& m = s.m;
   const MjbData& d = s.d;
   const int nv = s.nv, lane = s.lane;
-  mul_m_ctx(s, s.mv, s.search);
+  mulm();
   float q1 = 0.f, q2 = 0.f, q0 = 0.f;
   for (int i = lane; i < nv; i += 32) {
     q0 += s.gauss / float(nv);
@@ -222,9 +225,7 @@ __device__ void linesearch(SolverCtx& s) {
   s.qg[2] = warp_sum(q2);
   for (int k = lane; k < s.n; k += 32) {
     const int r = s.adr + k;
-    const float* J = d.efc_J + size_t(r) * nv;
-    float jv = 0.f;
-    for (int i = 0; i < nv; i++) jv += J[i] * s.search[i];
+    const float jv = rowdot(k);
     const float Jaref = d.efc_Jaref[r], D = d.efc_D[r];
     d.efc_jv[r] = jv;
     d.efc_quad[3 * r] = 0.5f * Jaref * Jaref * D;
@@ -293,7 +294,7 @@ __device__ void linesearch(SolverCtx& s) {
       }
       for (int t = 0; t < na; t++) {
         float g[3];
-        eval_pt3(s.qg, al[t], g);
+        evalg(s.qg, al[t], g);
         out[t][0] = g[0] + warp_sum(acc[t][0]);
         out[t][1] = g[1] + warp_sum(acc[t][1]);
         out[t][2] = g[2] + warp_sum(acc[t][2]);
@@ -352,6 +353,17 @@ __device__ void linesearch(SolverCtx& s) {
   }
   for (int k = lane; k < s.n; k += 32) d.efc_Jaref[s.adr + k] += s.alpha * d.efc_jv[s.adr + k];
   __syncwarp();
+}
+
+__device__ void linesearch(SolverCtx& s) {
+  linesearch_with(s, [&]() { mul_m_ctx(s, s.mv, s.search); },
+                  [&](int k) {
+                    const float* J = s.d.efc_J + size_t(s.adr + k) * s.nv;
+                    float jv = 0.f;
+                    for (int i = 0; i < s.nv; i++) jv += J[i] * s.search[i];
+                    return jv;
+                  },
+                  [](const float* q, float a, float* out) { eval_pt3(q, a, out); });
 }
 
 // solver.py:872-1000, any nv; hs: per-world nv*nv floats (the Newton Hessian and its factor);

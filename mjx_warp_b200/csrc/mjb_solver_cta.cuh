@@ -20,6 +20,8 @@
 // structure holds, and for the tensor-core assembly.
 #pragma once
 
+#include <type_traits>
+
 #include "mjb_solver.cuh"
 
 namespace mjb {
@@ -304,54 +306,61 @@ __device__ __noinline__ void cho_solve_cta(const float* L, int ld, int n, float*
 // of one Newton iteration outgrew the instruction cache (no_instruction stalls 2.4 cycles per issue
 // against 0.3, solver 21.1 against 13.0 ms).  Measured on the bin, Newton 10 iterations, whole step:
 // 4096 worlds 83.2 -> 16.5 ms, 300 worlds with the sparse mass matrix 12.4 -> 4.7 ms.
-constexpr int kSpTrees = 64;     // trees (bits of a mask)
-constexpr int kSpDofs = 512;     // 64 chunks of 8 dofs (bits of a mask)
-constexpr int kSpPanels = kSpDofs / 32;
-constexpr int kSpNodes = kSpTrees + kSpPanels;  // a tree's dofs within one panel
-constexpr int kSpRows = 736;     // rows with their trees in shared memory
-constexpr int kSpBlocks = 512;   // nonzero tree pairs of L
-constexpr int kSpSlots = 512;    // groups of up to 8 rows of a tree below a panel
-constexpr int kSpItems = 704;    // 8 x 8 tiles of L updated by earlier panels
-constexpr int kSpJ = 2048;       // floats of staged nonzero row entries
-constexpr int kSpL = 4096;       // floats of L kept in shared memory
+constexpr int kSpTrees = 64;  // trees (bits of a mask)
+// Capacities of the structure in shared memory, for models of up to kDofs dofs: kRows rows with
+// their trees, kBlocks nonzero tree pairs of L, kSlots groups of up to 8 rows of a tree below a
+// panel, kItems 8 x 8 tiles of L updated by earlier panels, kJ floats of staged nonzero row entries,
+// kL floats of L.  Large: 4 worlds of the 384-dof bin per SM (57 KB each); Small: 9 worlds of up to
+// 128 dofs (24 KB).
+struct SparseLarge {
+  static constexpr int kDofs = 512, kRows = 736, kBlocks = 512, kSlots = 512, kItems = 704, kJ = 2048, kL = 4096;
+};
+struct SparseSmall {
+  static constexpr int kDofs = 128, kRows = 192, kBlocks = 160, kSlots = 160, kItems = 192, kJ = 4, kL = 2560;
+};
 
 // One direction's schedule of the triangular solves: the nodes by dependency level, eight lanes
 // per node (32 for a node of more than 8 dofs), packed into warps.
+template <int NODES>
 struct SparseOrder {
-  uint8_t slot[4 * kSpNodes];   // node of each group of eight lanes, 255: none
-  uint8_t start[kSpNodes + 1];  // first warp of each level
+  uint8_t slot[4 * NODES];   // node of each group of eight lanes, 255: none
+  uint8_t start[NODES + 1];  // first warp of each level
   int levels;
 };
 
+template <class C>
 struct SparseShape {
+  static constexpr int kDofs = C::kDofs, kRows = C::kRows, kBlocks = C::kBlocks, kSlots = C::kSlots,
+                       kItems = C::kItems, kJ = C::kJ, kL = C::kL, kPanels = C::kDofs / 32,
+                       kNodes = kSpTrees + kPanels;  // nodes: a tree's dofs within one panel
   unsigned long long tmask[kSpTrees];      // trees u <= t with L(t, u) != 0, t itself among them
   unsigned long long tup[kSpTrees];        // trees t > u with L(t, u) != 0
-  unsigned long long cmask[kSpDofs / 8];   // 8-column chunks != 0 in each 8-row tile of L
-  unsigned long long ptrees[kSpPanels];    // trees with dofs in each 32-column panel
-  float cj[kSpJ];                          // staged row entries (tree u's, then tree t's)
-  float cl[kSpL];                          // L, each tree's rows over its nonzero columns
-  float sD[kSpRows];                       // D of the active rows, 0 elsewhere
-  float sF[kSpRows];                       // the rows' forces
+  unsigned long long cmask[kDofs / 8];   // 8-column chunks != 0 in each 8-row tile of L
+  unsigned long long ptrees[kPanels];    // trees with dofs in each 32-column panel
+  float cj[kJ];                          // staged row entries (tree u's, then tree t's)
+  float cl[kL];                          // L, each tree's rows over its nonzero columns
+  float sD[kRows];                       // D of the active rows, 0 elsewhere
+  float sF[kRows];                       // the rows' forces
   float* L;                                // cl, or efc_h when L does not fit there
   int rbase[kSpTrees];                     // a tree's first row in L and its row stride
-  uint32_t rlist[2 * kSpRows];             // each tree's rows, ascending: row | other tree << 16
-  uint32_t group[kSpDofs];                 // dofs of the panel coupled (transitively) with a dof
+  uint32_t rlist[2 * kRows];             // each tree's rows, ascending: row | other tree << 16
+  uint32_t group[kDofs];                 // dofs of the panel coupled (transitively) with a dof
   uint16_t rld[kSpTrees];
   uint16_t tadr[kSpTrees + 1];             // first dof of each tree
   uint16_t radr[kSpTrees + 1];             // first entry of each tree's rows in rlist
-  uint16_t rtree[kSpRows];                 // a row's trees: u | t << 8, u <= t (u == t: one tree)
+  uint16_t rtree[kRows];                 // a row's trees: u | t << 8, u <= t (u == t: one tree)
   uint16_t bst[kSpTrees + 1];              // a tree's first pair in blk / bcol
-  uint16_t blk[kSpBlocks];                 // nonzero tree pairs t << 8 | u, u <= t
-  uint16_t bcol[kSpBlocks];                // the pair's first column in its tree's rows of L
-  uint16_t pslot[kSpSlots];                // each panel's rows below that are != 0 in it: tree | 8-row group << 8
-  uint16_t padr[kSpPanels + 1];            // first entry of each panel in pslot
-  uint16_t iadr[kSpPanels + 1];            // first entry of each panel in item
-  uint32_t item[kSpItems];                 // a panel's updated 8 x 8 tiles: tree u | column group << 6 |
+  uint16_t blk[kBlocks];                 // nonzero tree pairs t << 8 | u, u <= t
+  uint16_t bcol[kBlocks];                // the pair's first column in its tree's rows of L
+  uint16_t pslot[kSlots];                // each panel's rows below that are != 0 in it: tree | 8-row group << 8
+  uint16_t padr[kPanels + 1];            // first entry of each panel in pslot
+  uint16_t iadr[kPanels + 1];            // first entry of each panel in item
+  uint32_t item[kItems];                 // a panel's updated 8 x 8 tiles: tree u | column group << 6 |
                                            // tree t << 11 | row group << 17, by u and column group
-  uint16_t nadr[kSpNodes + 1];             // first dof of each node
-  uint8_t ntree[kSpNodes];                 // its tree
-  uint8_t dtree[kSpDofs];                  // tree of each dof
-  SparseOrder fwd, bwd;
+  uint16_t nadr[kNodes + 1];             // first dof of each node
+  uint8_t ntree[kNodes];                 // its tree
+  uint8_t dtree[kDofs];                  // tree of each dof
+  SparseOrder<kNodes> fwd, bwd;
   int nblk, bad, compact;
   unsigned cnt[kSpTrees];
 
@@ -361,17 +370,22 @@ struct SparseShape {
   }
   __device__ __forceinline__ float* row(int i, int t) const { return L + rbase[t] + (i - tadr[t]) * rld[t]; }
 };
-constexpr int kSpFloats = int((sizeof(SparseShape) + 15) / 16 * 4);
+template <int NW>
+using SparseFor = SparseShape<std::conditional_t<NW == 1, SparseSmall, SparseLarge>>;
+template <class SH>
+constexpr int kSpFloats = int((sizeof(SH) + 15) / 16 * 4);
 
-__device__ __forceinline__ bool sparse_model(const MjbModel& m) {
-  return m.nblock >= 2 && m.nblock <= kSpTrees && m.nv <= kSpDofs;
+template <class SH>
+__host__ __device__ __forceinline__ bool sparse_model(const MjbModel& m) {
+  return m.nblock >= 2 && m.nblock <= kSpTrees && m.nv <= SH::kDofs;
 }
 
 __device__ __forceinline__ unsigned long long bits_below(int b) {  // bits 0 .. b - 1
   return b >= 64 ? ~0ull : (1ull << b) - 1ull;
 }
 // the dofs of panel c0 .. c0 + pn - 1 that lie in tree u, as a mask
-__device__ __forceinline__ unsigned panel_bits(const SparseShape& S, int u, int c0, int pn) {
+template <class SH>
+__device__ __forceinline__ unsigned panel_bits(const SH& S, int u, int c0, int pn) {
   const int q0 = max(int(S.tadr[u]) - c0, 0), q1 = min(int(S.tadr[u + 1]) - c0, pn);
   return unsigned(bits_below(q1) & ~bits_below(q0));
 }
@@ -379,14 +393,14 @@ __device__ __forceinline__ unsigned panel_bits(const SparseShape& S, int u, int 
 // Finds the structure of a world's n rows (J: n x nv dense) by a CTA of NW warps; false (in every
 // thread) when it does not fit the masks or lists, and the dense routines then run.  cw: floats per
 // row of cj (twice the largest tree), or 0 when the rows do not fit there.  H: the world's efc_h.
-template <int NW>
+template <int NW, class SH>
 __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int n, float* H,
-                                          SparseShape& S, int& cw, int warp, int lane) {
+                                          SH& S, int& cw, int warp, int lane) {
   const int nv = m.nv, nt = m.nblock, tid = warp * 32 + lane;
   constexpr int NT = NW * 32;
-  if (n > kSpRows) return false;
+  if (n > SH::kRows) return false;
   cw = 2 * m.block_max;
-  if (n * cw > kSpJ) cw = 0;
+  if (n * cw > SH::kJ) cw = 0;
   if (tid == 0) S.bad = 0;
 #pragma unroll 1
   for (int t = tid; t < nt; t += NT) {
@@ -487,7 +501,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
     int tot0, tot1;
     const int e0 = warp_excl_scan(__popcll(m0), lane, &tot0);
     const int e1 = warp_excl_scan(__popcll(m1), lane, &tot1) + tot0;
-    const bool fits = tot0 + tot1 <= kSpBlocks;
+    const bool fits = tot0 + tot1 <= SH::kBlocks;
     if (lane == 0) {
       S.nblk = tot0 + tot1;
       if (!fits) S.bad = 1;
@@ -517,7 +531,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
     const int z1 = lane + 32 < nt ? S.tadr[lane + 33] - S.tadr[lane + 32] : 0;
     int f0, f1;
     const int b0 = warp_excl_scan(w0 * z0, lane, &f0), b1 = warp_excl_scan(w1 * z1, lane, &f1) + f0;
-    const bool compact = f0 + f1 <= kSpL;
+    const bool compact = f0 + f1 <= SH::kL;
     if (lane == 0) {
       S.L = compact ? S.cl : H;
       S.compact = compact;
@@ -609,7 +623,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
 #pragma unroll 1
     for (int p = 0; p < n32; p++) {
       const int c1 = min(32 * p + 32, nv);
-      if (lane == 0) S.padr[p] = uint16_t(min(at, kSpSlots));
+      if (lane == 0) S.padr[p] = uint16_t(min(at, SH::kSlots));
 #pragma unroll 1
       for (int h = 0; h < 64; h += 32) {
         const int t = h + lane;
@@ -619,13 +633,13 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
         const int e = at + warp_excl_scan(z, lane, &tot);
 #pragma unroll 1
         for (int j = 0; j < z; j++)
-          if (e + j < kSpSlots) S.pslot[e + j] = uint16_t(t | (j << 8));
+          if (e + j < SH::kSlots) S.pslot[e + j] = uint16_t(t | (j << 8));
         at += tot;
       }
     }
     if (lane == 0) {
-      S.padr[n32] = uint16_t(min(at, kSpSlots));
-      if (at > kSpSlots) S.bad = 1;
+      S.padr[n32] = uint16_t(min(at, SH::kSlots));
+      if (at > SH::kSlots) S.bad = 1;
     }
   }
   if (warp == NW - 1) {  // the tiles that earlier panels update: the pairs with a common earlier tree
@@ -633,7 +647,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
 #pragma unroll 1
     for (int p = 0; p < n32; p++) {
       const int c0 = 32 * p, c1 = min(c0 + 32, nv);
-      if (lane == 0) S.iadr[p] = uint16_t(min(at, kSpItems));
+      if (lane == 0) S.iadr[p] = uint16_t(min(at, SH::kItems));
       if (p == 0) continue;
       const int tb = S.dtree[c0];
       const unsigned long long early = bits_below(tb + (S.tadr[tb] < c0 ? 1 : 0));
@@ -653,23 +667,24 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
             const int e = at + warp_excl_scan(z, lane, &tot);
 #pragma unroll 1
             for (int j = 0; j < z; j++)
-              if (e + j < kSpItems) S.item[e + j] = unsigned(u) | (unsigned(cg) << 6) | (unsigned(t) << 11) | (unsigned(j) << 17);
+              if (e + j < SH::kItems) S.item[e + j] = unsigned(u) | (unsigned(cg) << 6) | (unsigned(t) << 11) | (unsigned(j) << 17);
             at += tot;
           }
       }
     }
     if (lane == 0) {
-      S.iadr[n32] = uint16_t(min(at, kSpItems));
-      if (at > kSpItems) S.bad = 1;
+      S.iadr[n32] = uint16_t(min(at, SH::kItems));
+      if (at > SH::kItems) S.bad = 1;
     }
   }
   __syncthreads();
   if (S.bad) return false;
   // Levels: a node waits for every node of the trees its rows (forward) or columns (backward) couple
   // with, and for its own tree's previous node.  Warp 0 takes the forward order, warp 1 the other.
-  if (warp < 2) {
-    const bool bw = warp == 1;
-    SparseOrder& O = bw ? S.bwd : S.fwd;
+#pragma unroll 1
+  for (int dir = warp; dir < 2; dir += NW) {
+    const bool bw = dir == 1;
+    auto& O = bw ? S.bwd : S.fwd;
     int last[2], first[2], len[2];  // levels of the trees' last and first nodes to be solved
     unsigned long long dep[2];
 #pragma unroll
@@ -812,15 +827,60 @@ __device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned 
 // independent, so they are gathered; the chunks are those of the dense form); (ii) the diagonal
 // block gathered into T, factored by warp 0 group by group; (iii) the rows below solve against it,
 // a lane per row and up to eight columns of one tree in registers.
-template <int NW>
-__device__ __noinline__ void chol_cta_sparse(int n, float* T, const SparseShape& S, int warp, int lane) {
+template <int NW, class SH>
+__device__ __noinline__ void chol_cta_sparse(int n, float* T, const SH& S, int warp, int lane) {
   constexpr int TL = 36;
   const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll 1
   for (int c0 = 0; c0 < n; c0 += 32) {
     const int pn = min(32, n - c0), p = c0 >> 5;
     const int m0 = S.iadr[p], m1 = S.iadr[p + 1];
-    if (m1 > m0) {
+    if (NW == 1 && m1 > m0) {
+      // chol_blocked's trailing updates, panel by panel: four partial sums by column mod 4.  Lane:
+      // row g and columns t4, t4 + 4 of the tile.
+      for (int e = m0; e < m1; e++) {
+        const unsigned ia = S.item[e];
+        const int u = ia & 63, ta = (ia >> 11) & 63;
+        const int cb = max(int(S.tadr[u]), c0) + 8 * ((ia >> 6) & 31) + t4, ce = min(int(S.tadr[u + 1]), c0 + pn);
+        const int r = max(int(S.tadr[ta]), c0) + 8 * (ia >> 17) + g;
+        const bool kr = r < S.tadr[ta + 1], k0 = kr && cb < ce && cb <= r, k1 = kr && cb + 4 < ce && cb + 4 <= r;
+        const float* Lr = S.row(kr ? r : S.tadr[ta], ta);
+        const float* L0 = S.row(k0 ? cb : S.tadr[u], u);
+        const float* L1 = S.row(k1 ? cb + 4 : S.tadr[u], u);
+        float* C = const_cast<float*>(Lr) + S.col(ta, u) + cb - S.tadr[u];
+        float a0 = k0 ? C[0] : 0.f, a1 = k1 ? C[4] : 0.f;
+        float s[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+        int pv = -1;  // the earlier panel of the sums
+        for (unsigned long long b = S.tmask[u] & S.tmask[ta]; b; b &= b - 1ull) {
+          const int v = __ffsll(b) - 1, av = S.tadr[v], ev = min(int(S.tadr[v + 1]), c0);
+          if (av >= c0) break;
+          const int ct = S.col(ta, v) - av, cu = S.col(u, v) - av;
+          for (int k = av & ~3; k < ev; k += 4) {
+            if ((k >> 5) != pv) {
+              a0 -= (s[0] + s[1]) + (s[2] + s[3]);
+              a1 -= (z[0] + z[1]) + (z[2] + z[3]);
+#pragma unroll
+              for (int q = 0; q < 4; q++) s[q] = z[q] = 0.f;
+              pv = k >> 5;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              if (k + q >= av && k + q < ev) {
+                const float x = Lr[ct + k + q];
+                s[q] += x * L0[cu + k + q];
+                z[q] += x * L1[cu + k + q];
+              }
+            }
+          }
+        }
+        a0 -= (s[0] + s[1]) + (s[2] + s[3]);
+        a1 -= (z[0] + z[1]) + (z[2] + z[3]);
+        if (k0) C[0] = a0;
+        if (k1) C[4] = a1;
+      }
+      __syncwarp();
+    }
+    if (NW > 1 && m1 > m0) {
       const unsigned long long low = bits_below(c0 >> 3);
 #pragma unroll 1
       for (int e = m0 + 2 * warp; e < m1; e += 2 * NW) {
@@ -971,9 +1031,9 @@ __device__ __noinline__ void chol_cta_sparse(int n, float* T, const SparseShape&
 // solve's order: the part outside the 32-dof block first (forward: lane-strided partials added by
 // a 32-lane butterfly, formed by eight lanes per row; backward: one partial per warp of that form),
 // then the block's terms one by one.
-template <int NW>
+template <int NW, class SH>
 __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* y, float* z,
-                                                  const SparseShape& S, int warp, int lane) {
+                                                  const SH& S, int warp, int lane) {
   const int l8 = lane & 7;
 #pragma unroll 1
   for (int lev = 0; lev < S.fwd.levels; lev++) {  // L z = y
@@ -988,7 +1048,7 @@ __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* 
       const unsigned long long tm = any ? S.tmask[t] : 0ull;
       // trees with dofs before the block
       const int tb = S.dtree[c0];
-      const unsigned long long before = tm & bits_below(tb + (S.tadr[tb] < c0 ? 1 : 0));
+      const unsigned long long before = NW == 1 ? 0ull : tm & bits_below(tb + (S.tadr[tb] < c0 ? 1 : 0));
       float a = 0.f;
       const float* Lr = S.row(own ? r : i0, t);
       if (own && before) {
@@ -1030,11 +1090,11 @@ __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* 
       }
       float zi = own ? y[r] - a : 0.f;
       if (own)
-        for (unsigned long long b = tm & S.ptrees[c0 >> 5] & ~(1ull << t); b; b &= b - 1ull) {
-          const int u = __ffsll(b) - 1, au = S.tadr[u], end = S.tadr[u + 1];
+        for (unsigned long long b = NW == 1 ? tm : tm & S.ptrees[c0 >> 5] & ~(1ull << t); b; b &= b - 1ull) {
+          const int u = __ffsll(b) - 1, au = S.tadr[u], end = min(int(S.tadr[u + 1]), i0);
           const float* Lu = Lr + S.col(t, u) - au;
 #pragma unroll 1
-          for (int k = max(au, c0); k < end; k++) zi -= Lu[k] * z[k];
+          for (int k = NW == 1 ? au : max(au, c0); k < end; k++) zi -= Lu[k] * z[k];
         }
       const float* Lt = Lr + (any ? S.col(t, t) - S.tadr[t] : 0);
       const float diag = own ? Lt[r] : 1.f;
@@ -1066,7 +1126,7 @@ __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* 
       const unsigned long long up = own ? S.tup[t] : 0ull, in = S.ptrees[i0 >> 5];
       float s = 0.f;
       // rows outside the block: the node's own tree's (if it goes on) and the later trees'
-      const unsigned long long out = up | (own && S.tadr[t + 1] > c1 ? 1ull << t : 0ull);
+      const unsigned long long out = NW == 1 ? 0ull : up | (own && S.tadr[t + 1] > c1 ? 1ull << t : 0ull);
       if (out) {
         float acc[NW];  // the partials of the blocked form's warps
 #pragma unroll
@@ -1087,13 +1147,16 @@ __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* 
         for (int h = 0; h < NW; h++) s += acc[h];
       }
       float xi = own ? z[r] - s : 0.f;
+      // the block's later trees (one warp: every later dof), from the last dof
+      unsigned long long b = NW == 1 ? up | (own ? 1ull << t : 0ull) : up & in;
 #pragma unroll 1
-      for (unsigned long long b = up & in; b;) {  // the block's later trees, from the last dof
+      while (b) {
         const int u = 63 - __clzll(b), au = S.tadr[u], ld = S.rld[u];
         b &= ~(1ull << u);
         const float* Lu = S.L + S.rbase[u] + S.col(u, t) + ra;
 #pragma unroll 1
-        for (int i = min(int(S.tadr[u + 1]), c1) - 1; i >= au; i--) xi -= Lu[(i - au) * ld] * z[i];
+        for (int i = (NW == 1 ? int(S.tadr[u + 1]) : min(int(S.tadr[u + 1]), c1)) - 1; i >= max(au, i1); i--)
+          xi -= Lu[(i - au) * ld] * z[i];
       }
       const int lt = any ? S.rld[t] : 0;
       const float* Lt = S.L + S.rbase[t] + (own ? S.col(t, t) + ra : 0) - int(S.tadr[t]) * lt;
@@ -1125,8 +1188,9 @@ __device__ __noinline__ void cho_solve_cta_sparse(int n, float* x, const float* 
 __host__ __device__ __forceinline__ int tri(int i) { return i * (i + 1) / 2; }
 // the sparse structure, or (dense rows) each warp's row-compaction scratch
 __host__ __device__ __forceinline__ int cta_solver_union_floats(int nv, int nw, bool prec) {
-  const int dense = nw * 2 * round4i(nv);
-  return prec || dense > kSpFloats ? dense : kSpFloats;
+  const int sp = nw == 1 ? kSpFloats<SparseFor<1>> : kSpFloats<SparseFor<2>>;
+  const int dense = nw == 1 ? generic_nz_floats(nv) : nw * 2 * round4i(nv);
+  return prec || dense > sp ? dense : sp;
 }
 __host__ __device__ __forceinline__ int cta_solver_smem_base(int nv, int nw, bool prec) {
   return round4i(32 * nw + 32 * 36 + 32 + round4i(nv)) + cta_solver_union_floats(nv, nw, prec);
@@ -1252,7 +1316,8 @@ struct CtaSolver {
   bool sp = false;      // the world's sparsity is in S: nonzero trees and tiles only
   bool cleared = false; // the zeros of efc_h's lower triangle are written
   int cw = 0;           // floats per staged row in S->cj, 0: entries read from efc_J
-  SparseShape* S;
+  using SH = SparseFor<NW>;
+  SH* S;
   bool tc = false;  // FP32 form: the Hessian assembled on the tensor pipe (assemble_hessian_tc)
   float cost, prev_cost, gauss, grad_dot, search_dot, gtol, alpha, beta;
   float qg[3];
@@ -1325,8 +1390,31 @@ struct CtaSolver {
     return S->cj + k * cw + (tr == u ? 0 : S->tadr[u + 1] - S->tadr[u]);
   }
 
+  // J_k . x in column order (solve_generic's sum)
+  __device__ __forceinline__ float row_dot(int k, const float* x) const {
+    const int pr = S->rtree[k], u = pr & 255, t = pr >> 8;
+    float v = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < (u == t ? 1 : 2); q++) {
+      const int tr = q ? t : u, a = S->tadr[tr], z = S->tadr[tr + 1];
+      const float* e = row_entries(k, tr);
+#pragma unroll 2
+      for (int c = a; c < z; c++) v += e[c - a] * x[c];
+    }
+    return v;
+  }
+
   // out[r] = J_r . x - sub[r] for every row (warp per row); sub may be null
   __device__ void rows_dot(const float* x, float* out, const float* sub) {
+    if (sp && NW == 1) {
+#pragma unroll 1
+      for (int k = lane; k < n; k += 32) {
+        const float v = row_dot(k, x);
+        out[adr + k] = sub ? v - sub[adr + k] : v;
+      }
+      __syncwarp();
+      return;
+    }
     if (sp) {
       // Eight lanes per row over its trees' columns.  The dense form sums lane-strided partials
       // by a 32-lane butterfly; column c's partial belongs to lane c mod 32, so lane l of the eight
@@ -1701,8 +1789,8 @@ struct CtaSolver {
       } else {
         if (sp) {
           assemble_hessian_sparse();
-          chol_cta_sparse<NW>(nv, T, *S, warp, lane);
-        } else {
+          chol_cta_sparse<NW, SH>(nv, T, *S, warp, lane);
+        } else if constexpr (NW > 1) {
           if (tc) assemble_hessian_tc(H, nv);
           else assemble_hessian();
           chol_cta<NW>(H, nv, nv, T, warp, lane);
@@ -1713,13 +1801,40 @@ struct CtaSolver {
     if (warp == 0) {
       if (PREC) cho_solve_d_warp(Ld, rdg, nv, vd, Mgrad, grad, lane);
     }
-    if (!PREC && sp) cho_solve_cta_sparse<NW>(nv, Mgrad, grad, zv, *S, warp, lane);
-    else if (!PREC) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
+    if (!PREC && sp) cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
+    else if constexpr (!PREC && NW > 1) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
     __syncthreads();
   }
 
   // solver.py:737-869 with the iterative (:339-664) or parallel (:667-734) line search
   __device__ void linesearch() {
+    if constexpr (NW == 1) {  // solve_generic's own search
+      SolverCtx c{m, d, w, lane, nv, adr, n};
+      c.qacc = qacc;
+      c.Ma = Ma;
+      c.search = search;
+      c.mv = mv;
+      c.qfrc_smooth = qfrc_smooth;
+      c.gauss = gauss;
+      c.search_dot = search_dot;
+      c.alpha = alpha;
+      c.gtol = gtol;
+      // eval_pt3 with the multiply-adds that the compiler fuses in solve_generic written out: the
+      // two solvers give the same bits
+      linesearch_with(c, [&]() { mul_m(mv, search); }, [&](int k) { return row_dot(k, search); },
+                      [](const float* q, float a, float* out) {
+                        out[0] = __fadd_rn(__fmaf_rn(a, q[1], __fmul_rn(__fmul_rn(a, a), q[2])), q[0]);
+                        out[1] = __fmaf_rn(__fmul_rn(2.f, a), q[2], q[1]);
+                        out[2] = 2.f * q[2];
+                      });
+      alpha = c.alpha;
+      gtol = c.gtol;
+      for (int k = 0; k < 3; k++) qg[k] = c.qg[k];
+    } else {
+      linesearch_cta();
+    }
+  }
+  __device__ void linesearch_cta() {
     mul_m(mv, search);
     {
       float q[3] = {0.f, 0.f, 0.f};
@@ -1923,8 +2038,14 @@ struct CtaSolver {
 
   __device__ void run() {
     const float* ws = d.qacc_warmstart + W(w, nv);
-    if (!PREC && !tc && sparse_model(m))
-      sp = sparse_shape<NW>(m, d.efc_J + size_t(adr) * nv, n, H, *S, cw, warp, lane);
+    if constexpr (NW == 1) {  // solve_generic's arithmetic, which takes the worlds that do not fit
+      sp = sparse_shape<NW, SH>(m, d.efc_J + size_t(adr) * nv, n, H, *S, cw, warp, lane);
+      if (!sp) {
+        solve_generic(m, d, w, lane, H, nz, true);
+        return;
+      }
+    } else if (!PREC && !tc && sparse_model<SH>(m))
+      sp = sparse_shape<NW, SH>(m, d.efc_J + size_t(adr) * nv, n, H, *S, cw, warp, lane);
 #pragma unroll 1
     for (int i = tid; i < nv; i += NT) qacc[i] = ws[i];
     __syncthreads();
@@ -2016,7 +2137,7 @@ __device__ void solve_cta(const MjbModel& m, const MjbData& d, int w, float* sme
   s.zv = smem + 32 * NW + 32 * 36 + 32;
   float* part = smem + round4i(32 * NW + 32 * 36 + 32 + round4i(nv));  // structure or scratch
   s.nz = part + warp * 2 * round4i(nv);
-  s.S = reinterpret_cast<SparseShape*>(part);
+  s.S = reinterpret_cast<SparseFor<NW>*>(part);
   s.Ld = PREC ? reinterpret_cast<double*>(smem + cta_solver_smem_base(nv, NW, PREC)) : nullptr;
   s.vd = PREC ? s.Ld + tri(nv) : nullptr;
   s.rdg = PREC ? s.vd + nv : nullptr;

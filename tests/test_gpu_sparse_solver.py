@@ -78,3 +78,31 @@ def test_factor_of_the_hessian(name, warps):
     L = np.tril(d.efc.h[w].cpu().numpy().astype(np.float64))
     r = np.linalg.norm(L @ L.T - H) / np.linalg.norm(H)
     assert r < 2 * (mjm.nv + 1) * 2.0 ** -24, (w, r)
+
+
+@pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres16", "humanoid_spheres"])
+def test_one_warp_form_equals_plain(name):
+  """Up to 128 dofs the chosen form solves a world by one warp over the nonzero trees in the plain
+  form's arithmetic: equal values, whether the world fits the structure or (more than 192 rows: the
+  16 spheres in one heap) takes the generic solver."""
+  mjm, q, v, u, cap = case(name)
+  mjm.opt.iterations = 10
+  if name == "spheres16":
+    x = q.reshape(5, -1, 7)
+    x[1:3, :, :3] = 0.15 + 0.05 * (x[1:3, :, :3] - x[1:3, :1, :3])
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  out = {}
+  for form in (1, 0):
+    d = device_data(mjm, q, v, u, nconmax=800 * nworld, njmax=cap * nworld)
+    mjw.forward(m, d, fused=form)
+    torch.cuda.synchronize()
+    assert np.all(mjw.world_status(d) == 0)
+    out[form] = d
+  n = world_rows(out[1], "efc")[0]
+  assert name != "spheres16" or n.max() > 192 > n.min()
+  for f in ("qacc", "qfrc_constraint"):
+    assert torch.equal(getattr(out[1], f), getattr(out[0], f)), f
+  for f in ("cost", "Ma", "h"):
+    a, b = getattr(out[1].efc, f), getattr(out[0].efc, f)
+    assert torch.equal(a.tril(), b.tril()) if f == "h" else torch.equal(a, b), f
