@@ -201,6 +201,13 @@ __device__ __forceinline__ void eval_pt3(const float* q, float a, float* out) {
   out[1] = 2.f * a * q[2] + q[1];
   out[2] = 2.f * q[2];
 }
+// eval_pt3 with its fused multiply-adds written out, so that the rounding of the costs (the line
+// search compares them) does not change with the code around it
+__device__ __forceinline__ void eval_pt3_fma(const float* q, float a, float* out) {
+  out[0] = __fadd_rn(__fmaf_rn(a, q[1], __fmul_rn(__fmul_rn(a, a), q[2])), q[0]);
+  out[1] = __fmaf_rn(__fmul_rn(2.f, a), q[2], q[1]);
+  out[2] = 2.f * q[2];
+}
 __device__ __forceinline__ bool in_bracket(const float* x, const float* y) {
   return (x[1] < y[1] && y[1] < 0.f) || (x[1] > y[1] && y[1] > 0.f);
 }
@@ -478,22 +485,29 @@ __device__ __noinline__ void solve_generic(const MjbModel& m, const MjbData& d, 
 // ------------------------------------------------------------------------------------------
 // Solver for nv <= 32: lane i owns dof i, so every per-dof vector (qacc, Ma, grad, Mgrad, search,
 // mv, ...) lives in one register per lane; qM, the constraint Jacobian rows (when a world has at
-// most kSolverRows rows) and the Hessian factor live in the warp's shared-memory slice; per-row
+// most staged_rows(nv) rows) and the Hessian factor live in the warp's shared-memory slice; per-row
 // scalars stay in the flat efc arrays, each touched only by the lane that owns the row.
 
-#ifndef MJB_JROWS
-#define MJB_JROWS 32
-#endif
-constexpr int kSolverRows = MJB_JROWS;
+constexpr int kLaneRows = 32;      // staged rows with one row per lane
+constexpr int kSolverFloats = 2854;  // per warp at 5 CTAs of 4 warps per SM (228 KB, 1 KB reserved per CTA)
 
 __host__ __device__ __forceinline__ int round4(int x) { return (x + 3) & ~3; }
 // Per-warp layout, every part 16-byte aligned, every matrix row tile_ld(nv) floats with the
-// columns from nv to the next multiple of 4 zero: Ls (the factor tile, nv rows) | Js (kSolverRows
-// rows) | Ms (qM, nv rows) | vs (32) | F (kSolverRows).  The tile comes first so the fused step can
+// columns from nv to the next multiple of 4 zero: Ls (the factor tile, nv rows) | Js (staged_rows
+// rows) | Ms (qM, nv rows) | vs (32) | F (staged_rows).  The tile comes first so the fused step can
 // use it for the mass-matrix factorisations too.  Lanes read their own rows as float4 without bank
 // conflicts (see tile_ld).
+// Rows that are staged: up to 64 (two per lane) as far as five CTAs still fit an SM (45 at nv = 27,
+// 64 up to nv = 20), at least 32.  A humanoid world with 33 to 45 rows was the last to finish at any batch
+// size: its rows read through L1, line search scalars included, and its Hessian refactored in
+// every iteration, it took 605 k cycles against 100 k for the mean world (128 worlds, Newton 10).
+__host__ __device__ __forceinline__ int staged_rows(int nv) {
+  const int spare = kSolverFloats - 4 - 2 * tile_floats(nv) - 32;
+  const int r = spare / (tile_ld(nv) + 1);
+  return r < kLaneRows ? kLaneRows : (r > 64 ? 64 : r);
+}
 __host__ __device__ __forceinline__ size_t solver_smem_floats(int nv) {
-  return size_t(round4(2 * tile_floats(nv) + kSolverRows * tile_ld(nv) + 32 + kSolverRows));
+  return size_t(round4(2 * tile_floats(nv) + staged_rows(nv) * tile_ld(nv) + 32 + round4(staged_rows(nv))));
 }
 
 // sum_j a_j b_j over the first 4 * nq columns of two 16-byte aligned rows (four partial sums)
@@ -521,13 +535,14 @@ struct Small {
   int ld, nq;                   // staged row stride and float4 count per row (4 * nq >= nv)
   bool staged;                  // J rows copied to shared memory (else read from efc_J)
   bool own;
-  // With staged rows (n <= 32) lane k owns row k and keeps its scalars in registers; the flat
-  // efc arrays are then only written (they stay the observable outputs).
-  float rJaref = 0.f, rjv = 0.f, rD = 0.f, rq0 = 0.f, rq1 = 0.f, rq2 = 0.f;
-  int ract = 0;
+  // With staged rows lane k owns row k (and row k + 32) and keeps their scalars in registers; the
+  // flat efc arrays are then only written (they stay the observable outputs).
+  float rJaref[2] = {0.f, 0.f}, rjv[2] = {0.f, 0.f}, rD[2] = {0.f, 0.f};
+  float rq0[2] = {0.f, 0.f}, rq1[2] = {0.f, 0.f}, rq2[2] = {0.f, 0.f};
+  int ract[2] = {0, 0};
   bool reuse = false;           // keep the factor of H while the active set is unchanged
   bool factored = false;        // Ls holds the factor of H for the active set factored_mask
-  unsigned factored_mask = 0u;
+  unsigned factored_mask = 0u, factored_mask1 = 0u;  // of rows 0 .. 31 and 32 .. 63
   float *Ms, *Ls, *vs, *F;
   double* Ld = nullptr;         // precision form: the FP64 factor tile
   const float* J;
@@ -550,12 +565,24 @@ struct Small {
     vs[lane] = own ? v : 0.f;
     __syncwarp();
   }
-  template <bool ST>
+  template <int ST>
   __device__ __forceinline__ float rowdot(int k) const {
     const float* Jr = J + size_t(k) * ldj;
-    if (ST) return dotq(Jr, vs, nq);
+    if (ST == 1) return dotq(Jr, vs, nq);
     float s = 0.f;
-    for (int j = 0; j < nv; j++) s += Jr[j] * vs[j];
+    if constexpr (ST == 2) {  // in column order, as the rows that are not staged
+      const float4* a4 = reinterpret_cast<const float4*>(Jr);
+      const float4* b4 = reinterpret_cast<const float4*>(vs);
+      for (int q = 0; q < nq; q++) {  // the columns from nv on are zero
+        const float4 x = a4[q], y = b4[q];
+        s += x.x * y.x;
+        s += x.y * y.y;
+        s += x.z * y.z;
+        s += x.w * y.w;
+      }
+    } else {
+      for (int j = 0; j < nv; j++) s += Jr[j] * vs[j];
+    }
     return s;
   }
 };
@@ -635,7 +662,7 @@ __device__ __forceinline__ void hessian_tc(const float* Ms, const float* Js, int
 // solution.  Staged Jacobian rows are read as float4 broadcasts.
 // TC (staged rows only): H is assembled by hessian_tc on the tensor pipe instead; ix is 32 ints
 // of warp scratch for its row list.
-template <bool PREC, bool ST, bool TC = false>
+template <bool PREC, int ST, bool TC = false>
 __device__ __forceinline__ float newton_direction(const float* Ms, int ld, const float* J, int ldj,
                                                const float* C, const int* act,
                                                const float* D, int n, float* Ls, int nv,
@@ -643,7 +670,7 @@ __device__ __forceinline__ float newton_direction(const float* Ms, int ld, const
                                                double* Ld = nullptr, int* ix = nullptr) {
   const int nq = (nv + 3) >> 2;
   const bool own = lane < nv;
-  if (TC && ST && refactor) {  // n <= 32: lane k owns row k; list the rows with a nonzero coefficient
+  if (TC && ST == 1 && refactor) {  // n <= 32: lane k owns row k; list the rows with a nonzero coefficient
     const bool on = lane < n && C[lane] != 0.f;
     const unsigned mk = __ballot_sync(WARP_FULL, on);
     if (on) ix[__popc(mk & ((1u << lane) - 1u))] = lane;
@@ -672,42 +699,45 @@ __device__ __forceinline__ float newton_direction(const float* Ms, int ld, const
       // staged rows (n <= 32, zero-padded, 16-byte aligned): the rows with c != 0 taken from a
       // ballot mask in increasing order, two per pass (each h[j] still adds the rows' terms in
       // row order)
-      unsigned mk = __ballot_sync(WARP_FULL, lane < n && C[lane] != 0.f);
-      while (mk) {
-        const int k0 = __ffs(mk) - 1;
-        mk &= mk - 1u;
-        const float* J0 = J + k0 * ldj;
-        const float a0 = own ? C[k0] * J0[lane] : 0.f;
-        const float4* A4 = reinterpret_cast<const float4*>(J0);
-        if (mk) {
-          const int k1 = __ffs(mk) - 1;
+#pragma unroll 1
+      for (int base = 0; base < (ST == 2 ? 64 : 32); base += 32) {
+        unsigned mk = __ballot_sync(WARP_FULL, base + lane < n && C[base + lane] != 0.f);
+        while (mk) {
+          const int k0 = base + __ffs(mk) - 1;
           mk &= mk - 1u;
-          const float* J1 = J + k1 * ldj;
-          const float a1 = own ? C[k1] * J1[lane] : 0.f;
-          const float4* B4 = reinterpret_cast<const float4*>(J1);
+          const float* J0 = J + k0 * ldj;
+          const float a0 = own ? C[k0] * J0[lane] : 0.f;
+          const float4* A4 = reinterpret_cast<const float4*>(J0);
+          if (mk) {
+            const int k1 = base + __ffs(mk) - 1;
+            mk &= mk - 1u;
+            const float* J1 = J + k1 * ldj;
+            const float a1 = own ? C[k1] * J1[lane] : 0.f;
+            const float4* B4 = reinterpret_cast<const float4*>(J1);
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            if (q < nq) {
-              const float4 u = A4[q], v = B4[q];
-              h[4 * q] += a0 * u.x;
-              h[4 * q + 1] += a0 * u.y;
-              h[4 * q + 2] += a0 * u.z;
-              h[4 * q + 3] += a0 * u.w;
-              h[4 * q] += a1 * v.x;
-              h[4 * q + 1] += a1 * v.y;
-              h[4 * q + 2] += a1 * v.z;
-              h[4 * q + 3] += a1 * v.w;
+            for (int q = 0; q < 8; q++) {
+              if (q < nq) {
+                const float4 u = A4[q], v = B4[q];
+                h[4 * q] += a0 * u.x;
+                h[4 * q + 1] += a0 * u.y;
+                h[4 * q + 2] += a0 * u.z;
+                h[4 * q + 3] += a0 * u.w;
+                h[4 * q] += a1 * v.x;
+                h[4 * q + 1] += a1 * v.y;
+                h[4 * q + 2] += a1 * v.z;
+                h[4 * q + 3] += a1 * v.w;
+              }
             }
-          }
-        } else {
+          } else {
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            if (q < nq) {
-              const float4 u = A4[q];
-              h[4 * q] += a0 * u.x;
-              h[4 * q + 1] += a0 * u.y;
-              h[4 * q + 2] += a0 * u.z;
-              h[4 * q + 3] += a0 * u.w;
+            for (int q = 0; q < 8; q++) {
+              if (q < nq) {
+                const float4 u = A4[q];
+                h[4 * q] += a0 * u.x;
+                h[4 * q + 1] += a0 * u.y;
+                h[4 * q + 2] += a0 * u.z;
+                h[4 * q + 3] += a0 * u.w;
+              }
             }
           }
         }
@@ -753,22 +783,26 @@ __device__ __forceinline__ float ls_sum(float base, float x, bool prec) {
 }
 
 // solver.py:75-173
-template <bool ST>
+template <int ST>
 __device__ void small_update_constraint(Small& s) {
   const MjbData& d = s.d;
   s.prev_cost = s.cost;
   float c = 0.f;
   if (ST) {
-    if (s.lane < s.n) {
-      const int r = s.adr + s.lane;
-      const float Jaref = s.rJaref, D = s.rD;
-      const int active = Jaref < 0.f;
-      s.ract = active;
-      d.efc_active[r] = active;
-      const float f = active ? -1.f * D * Jaref : 0.f;
-      d.efc_force[r] = f;
-      s.F[s.lane] = f;
-      if (active) c += 0.5f * D * Jaref * Jaref;
+#pragma unroll
+    for (int h = 0; h < ST; h++) {
+      const int k = s.lane + 32 * h;
+      if (k < s.n) {
+        const int r = s.adr + k;
+        const float Jaref = s.rJaref[h], D = s.rD[h];
+        const int active = Jaref < 0.f;
+        s.ract[h] = active;
+        d.efc_active[r] = active;
+        const float f = active ? -1.f * D * Jaref : 0.f;
+        d.efc_force[r] = f;
+        s.F[k] = f;
+        if (active) c += 0.5f * D * Jaref * Jaref;
+      }
     }
   } else {
     for (int k = s.lane; k < s.n; k += 32) {
@@ -796,7 +830,7 @@ __device__ void small_update_constraint(Small& s) {
 }
 
 // solver.py:176-312
-template <bool PREC, bool ST, bool CG, bool TC>
+template <bool PREC, int ST, bool CG, bool TC>
 __device__ void small_update_gradient(Small& s) {
   const MjbModel& m = s.m;
   const MjbData& d = s.d;
@@ -815,14 +849,18 @@ __device__ void small_update_gradient(Small& s) {
   }
   // H depends on the solve's inputs only through the active set, so with s.reuse the factor of
   // the previous call is kept (bit-identical) while the set of active rows is unchanged; rows
-  // past the first 32 are not tracked, so such worlds refactor every time.  Without s.reuse every
+  // past the staged ones are not tracked, so such worlds refactor every time.  Without s.reuse every
   // call refactors, as the reference does.
-  constexpr bool staged = ST;  // unstaged rows keep F in efc_force, which must survive
+  constexpr bool staged = ST != 0;  // unstaged rows keep F in efc_force, which must survive
   const unsigned mask = __ballot_sync(
-      WARP_FULL, lane < s.n && (staged ? s.ract != 0 : d.efc_active[s.adr + lane] != 0));
-  const bool refactor = !s.reuse || !s.factored || s.n > 32 || mask != s.factored_mask;
+      WARP_FULL, lane < s.n && (staged ? s.ract[0] != 0 : d.efc_active[s.adr + lane] != 0));
+  const unsigned mask1 = ST == 2 ? __ballot_sync(WARP_FULL, lane + 32 < s.n && s.ract[1] != 0) : 0u;
+  const bool refactor = !s.reuse || !s.factored || s.n > 32 * (ST == 2 ? 2 : 1) || mask != s.factored_mask ||
+                        (ST == 2 && mask1 != s.factored_mask1);
   if (refactor && staged) {  // coefficient of each row in J^T D J: D when active, else 0
-    if (lane < s.n) s.F[lane] = s.ract ? s.rD : 0.f;
+#pragma unroll
+    for (int h = 0; h < ST; h++)
+      if (lane + 32 * h < s.n) s.F[lane + 32 * h] = s.ract[h] ? s.rD[h] : 0.f;
     __syncwarp();
   }
   s.Mgrad = newton_direction<PREC, ST, TC>(s.Ms, s.ld, s.J, s.ldj, staged ? s.F : nullptr,
@@ -830,10 +868,11 @@ __device__ void small_update_gradient(Small& s) {
                              refactor, s.Ld, reinterpret_cast<int*>(s.vs));
   s.factored = true;
   s.factored_mask = mask;
+  s.factored_mask1 = mask1;
 }
 
 // solver.py:737-869
-template <bool PREC, bool ST, bool LSP>
+template <bool PREC, int ST, bool LSP>
 __device__ void small_linesearch(Small& s) {
   const MjbModel& m = s.m;
   const MjbData& d = s.d;
@@ -842,7 +881,9 @@ __device__ void small_linesearch(Small& s) {
   // f(Jaref, jv, quad0, quad1, quad2) for each of this lane's rows (registers when staged)
   auto rows = [&](auto&& f) {
     if (ST) {
-      if (lane < s.n) f(s.rJaref, s.rjv, s.rq0, s.rq1, s.rq2);
+#pragma unroll
+      for (int h = 0; h < ST; h++)
+        if (lane + 32 * h < s.n) f(s.rJaref[h], s.rjv[h], s.rq0[h], s.rq1[h], s.rq2[h]);
     } else {
       for (int k = lane; k < s.n; k += 32) {
         const int r = s.adr + k;
@@ -862,18 +903,22 @@ __device__ void small_linesearch(Small& s) {
   }
   s.publish(s.search);
   if (ST) {
-    if (lane < s.n) {
-      const int r = s.adr + lane;
-      const float jv = s.template rowdot<ST>(lane);
-      const float Jaref = s.rJaref, D = s.rD;
-      s.rjv = jv;
-      s.rq0 = 0.5f * Jaref * Jaref * D;
-      s.rq1 = jv * Jaref * D;
-      s.rq2 = 0.5f * jv * jv * D;
-      d.efc_jv[r] = jv;
-      d.efc_quad[3 * r] = s.rq0;
-      d.efc_quad[3 * r + 1] = s.rq1;
-      d.efc_quad[3 * r + 2] = s.rq2;
+#pragma unroll
+    for (int h = 0; h < ST; h++) {
+      const int k = lane + 32 * h;
+      if (k < s.n) {
+        const int r = s.adr + k;
+        const float jv = s.template rowdot<ST>(k);
+        const float Jaref = s.rJaref[h], D = s.rD[h];
+        s.rjv[h] = jv;
+        s.rq0[h] = 0.5f * Jaref * Jaref * D;
+        s.rq1[h] = jv * Jaref * D;
+        s.rq2[h] = 0.5f * jv * jv * D;
+        d.efc_jv[r] = jv;
+        d.efc_quad[3 * r] = s.rq0[h];
+        d.efc_quad[3 * r + 1] = s.rq1[h];
+        d.efc_quad[3 * r + 2] = s.rq2[h];
+      }
     }
   } else {
     for (int k = lane; k < s.n; k += 32) {
@@ -933,7 +978,7 @@ __device__ void small_linesearch(Small& s) {
         for (int t = 0; t < na; t++) {
           if (jaref + al[t] * jv < 0.f) {
             float p[3];
-            eval_pt3(q, al[t], p);
+            eval_pt3_fma(q, al[t], p);
             acc[t][0] += p[0];
             acc[t][1] += p[1];
             acc[t][2] += p[2];
@@ -942,7 +987,7 @@ __device__ void small_linesearch(Small& s) {
       });
       for (int t = 0; t < na; t++) {
         float g[3];
-        eval_pt3(s.qg, al[t], g);
+        eval_pt3_fma(s.qg, al[t], g);
         out[t][0] = ls_sum(g[0], acc[t][0], prec);
         out[t][1] = ls_sum(g[1], acc[t][1], prec);
         out[t][2] = ls_sum(g[2], acc[t][2], prec);
@@ -998,10 +1043,12 @@ __device__ void small_linesearch(Small& s) {
     s.Ma += s.alpha * s.mv;
   }
   if (ST) {
-    if (lane < s.n) {
-      s.rJaref += s.alpha * s.rjv;
-      d.efc_Jaref[s.adr + lane] = s.rJaref;
-    }
+#pragma unroll
+    for (int h = 0; h < ST; h++)
+      if (lane + 32 * h < s.n) {
+        s.rJaref[h] += s.alpha * s.rjv[h];
+        d.efc_Jaref[s.adr + lane + 32 * h] = s.rJaref[h];
+      }
   } else {
     for (int k = lane; k < s.n; k += 32) d.efc_Jaref[s.adr + k] += s.alpha * d.efc_jv[s.adr + k];
   }
@@ -1009,9 +1056,9 @@ __device__ void small_linesearch(Small& s) {
 }
 
 // The iterations of solve_small once the world's rows are placed.  ST: rows staged in shared
-// memory (n <= kSolverRows); CG: the CG solver (else Newton); LSP: the parallel line search (else
+// memory (1: n <= 32, one row per lane; 2: n <= staged_rows(nv), two per lane); CG: the CG solver (else Newton); LSP: the parallel line search (else
 // the iterative one) -- compile-time choices, so that each path's code is straight.
-template <bool PREC, bool ST, bool CG, bool LSP, bool TC>
+template <bool PREC, int ST, bool CG, bool LSP, bool TC>
 __device__ void solve_small_run(Small& s) {
   const MjbModel& m = s.m;
   const MjbData& d = s.d;
@@ -1020,10 +1067,14 @@ __device__ void solve_small_run(Small& s) {
   s.cost = __int_as_float(0x7f800000);
   s.publish(s.qacc);
   if (ST) {
-    if (lane < n) {
-      s.rD = d.efc_D[adr + lane];
-      s.rJaref = s.template rowdot<ST>(lane) - d.efc_aref[adr + lane];
-      d.efc_Jaref[adr + lane] = s.rJaref;
+#pragma unroll
+    for (int h = 0; h < ST; h++) {
+      const int k = lane + 32 * h;
+      if (k < n) {
+        s.rD[h] = d.efc_D[adr + k];
+        s.rJaref[h] = s.template rowdot<ST>(k) - d.efc_aref[adr + k];
+        d.efc_Jaref[adr + k] = s.rJaref[h];
+      }
     }
   } else {
     for (int k = lane; k < n; k += 32) d.efc_Jaref[adr + k] = s.template rowdot<ST>(k) - d.efc_aref[adr + k];
@@ -1103,12 +1154,12 @@ __device__ void solve_small(const MjbModel& m, const MjbData& d, int w, int lane
   s.Ls = sm;
   if (PREC) s.Ld = reinterpret_cast<double*>(sm + solver_smem_floats(nv));
   float* Js = sm + tile_floats(nv);
-  s.Ms = Js + kSolverRows * s.ld;
+  s.Ms = Js + staged_rows(nv) * s.ld;
   s.vs = s.Ms + tile_floats(nv);
   s.F = s.vs + 32;
   const int ncol = 4 * s.nq;  // staged columns: nv, zero padded to a multiple of 4
   const float* Jg = d.efc_J + size_t(adr) * nv;
-  if (n <= kSolverRows) {
+  if (n <= staged_rows(nv)) {
     copy_rows(Jg, nv, Js, s.ld, n, nv, ncol, lane);  // rows zero padded for float4 reads
     s.J = Js;
     s.ldj = s.ld;
@@ -1129,16 +1180,23 @@ __device__ void solve_small(const MjbModel& m, const MjbData& d, int w, int lane
   s.qg[0] = s.qg[1] = s.qg[2] = 0.f;
   __syncwarp();
   const bool cg = m.solver == 1, lsp = m.ls_parallel != 0;
-  if (s.staged) {
-    if (!cg && !lsp) solve_small_run<PREC, true, false, false, TC>(s);
-    else if (!cg) solve_small_run<PREC, true, false, true, TC>(s);
-    else if (!lsp) solve_small_run<PREC, true, true, false, TC>(s);
-    else solve_small_run<PREC, true, true, true, TC>(s);
+  if (n <= kLaneRows) {
+    if (!cg && !lsp) solve_small_run<PREC, 1, false, false, TC>(s);
+    else if (!cg) solve_small_run<PREC, 1, false, true, TC>(s);
+    else if (!lsp) solve_small_run<PREC, 1, true, false, TC>(s);
+    else solve_small_run<PREC, 1, true, true, TC>(s);
+  } else if (s.staged && !cg && !lsp) {
+    solve_small_run<PREC, 2, false, false, TC>(s);
   } else {
-    if (!cg && !lsp) solve_small_run<PREC, false, false, false, TC>(s);
-    else if (!cg) solve_small_run<PREC, false, false, true, TC>(s);
-    else if (!lsp) solve_small_run<PREC, false, true, false, TC>(s);
-    else solve_small_run<PREC, false, true, true, TC>(s);
+    if (s.staged) {  // the rarer searches read their rows from efc_J
+      s.J = Jg;
+      s.ldj = nv;
+      s.F = d.efc_force + adr;
+    }
+    if (!cg && !lsp) solve_small_run<PREC, 0, false, false, TC>(s);
+    else if (!cg) solve_small_run<PREC, 0, false, true, TC>(s);
+    else if (!lsp) solve_small_run<PREC, 0, true, false, TC>(s);
+    else solve_small_run<PREC, 0, true, true, TC>(s);
   }
 }
 

@@ -1819,14 +1819,9 @@ struct CtaSolver {
       c.search_dot = search_dot;
       c.alpha = alpha;
       c.gtol = gtol;
-      // eval_pt3 with the multiply-adds that the compiler fuses in solve_generic written out: the
-      // two solvers give the same bits
+      // the smooth part as the compiler fuses it in solve_generic: the two give the same bits
       linesearch_with(c, [&]() { mul_m(mv, search); }, [&](int k) { return row_dot(k, search); },
-                      [](const float* q, float a, float* out) {
-                        out[0] = __fadd_rn(__fmaf_rn(a, q[1], __fmul_rn(__fmul_rn(a, a), q[2])), q[0]);
-                        out[1] = __fmaf_rn(__fmul_rn(2.f, a), q[2], q[1]);
-                        out[2] = 2.f * q[2];
-                      });
+                      [](const float* q, float a, float* out) { eval_pt3_fma(q, a, out); });
       alpha = c.alpha;
       gtol = c.gtol;
       for (int k = 0; k < 3; k++) qg[k] = c.qg[k];
