@@ -81,9 +81,11 @@ __device__ __forceinline__ void copy_qacc_smooth(const MjbModel& m, const MjbDat
   __syncwarp();
 }
 
-// the solver needs up to 128 registers; every other stage is held to 64 for occupancy
+// the solver needs up to 128 registers; make_constraint's lanes hold a contact each and need 80 (6
+// CTAs per SM: the fastest of 5, 6 and 8 on 8192 and on 32768 humanoid worlds, by 1 %); every other
+// stage is held to 64 for occupancy
 template <int STAGE>
-__global__ void __launch_bounds__(128, STAGE == S_SOLVE ? MJB_MINB : MJB_MINB_STAGE)
+__global__ void __launch_bounds__(128, STAGE == S_SOLVE ? MJB_MINB : (STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB_STAGE))
     k_stage(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int smem_per_warp) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;

@@ -502,6 +502,20 @@ __device__ void collision(const MjbModel& m, const MjbData& d, int w, int lane, 
   primitive_narrowphase(m, d, w, lane);
 }
 
+// the dofs [a, z) of the bodies under root body `root` (the world's: none)
+__device__ __forceinline__ void root_dofs(const MjbModel& m, int root, int& a, int& z) {
+  a = z = 0;
+  if (root == 0) return;
+  const int e = m.body_subtreeend[root];
+  for (int b = root; b < e; b++) {  // the bodies' dofs are consecutive
+    const int n = m.body_dofnum[b];
+    if (n > 0) {
+      if (z == 0) a = m.body_dofadr[b];
+      z = m.body_dofadr[b] + n;
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // constraint.py:22-73
 __device__ void update_efc_row(const MjbModel& m, const MjbData& d, int r, float pos_aref,
@@ -610,57 +624,137 @@ __device__ void make_constraint(const MjbModel& m, const MjbData& d, int w, int 
       run += __popc(mask);
     }
   }
-  // contact rows: lanes over dofs build the 4 pyramid rows of one contact at a time
+  // Contact rows: lanes over dofs build the 4 pyramid rows of one contact at a time.  What a contact
+  // needs is loaded by one lane per contact beforehand (its chain of dependent loads, geom to body to
+  // root to centre of mass, is waited out once per 32 contacts) and broadcast by shuffles; the rows'
+  // scalars are formed for eight contacts at once, a lane per row.
   if (ncact > 0) {
     const float* cdof = d.cdof + W(w, 6 * nv);
     const float* sc = d.subtree_com + W(w, 3 * m.nbody);
-    int r = adr + nlim;
-    for (int k = 0; k < nc; k++) {
-      const int c = ca + k;
-      if (!(d.contact_dim[c] == 3 && (d.contact_dist[c] - d.contact_includemargin[c]) < 0.f)) continue;
-      const float pos = d.contact_dist[c] - d.contact_includemargin[c];
-      const int b1 = m.geom_bodyid[d.contact_geom[2 * c]], b2 = m.geom_bodyid[d.contact_geom[2 * c + 1]];
-      const float* fr = d.contact_frame + 9 * c;
-      const float* fri = d.contact_friction + 5 * c;
-      const f3 cp = ld3(d.contact_pos + 3 * c);
-      const f3 off1 = cp - ld3(sc + 3 * m.body_rootid[b1]);
-      const f3 off2 = cp - ld3(sc + 3 * m.body_rootid[b2]);
-      float jq[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int i = lane; i < nv; i += 32) {
-        const s6 cd = ld6(cdof + 6 * i);
-        const f3 ang{cd.v[0], cd.v[1], cd.v[2]}, lin{cd.v[3], cd.v[4], cd.v[5]};
-        const int db = m.dof_bodyid[i];
-        // constraint.py:76-101: the dof moves body b iff its body is an ancestor-or-self of b
-        const float in1 = (db != 0 && db <= b1 && b1 < m.body_subtreeend[db]) ? 1.f : 0.f;
-        const float in2 = (db != 0 && db <= b2 && b2 < m.body_subtreeend[db]) ? 1.f : 0.f;
-        const f3 j1 = (lin + cross(ang, off1)) * in1;
-        const f3 j2 = (lin + cross(ang, off2)) * in2;
-        const f3 jd = j2 - j1;
-        const float diff0 = fr[0] * jd.x + fr[1] * jd.y + fr[2] * jd.z;
-        const float diff1 = fr[3] * jd.x + fr[4] * jd.y + fr[5] * jd.z;
-        const float diff2 = fr[6] * jd.x + fr[7] * jd.y + fr[8] * jd.z;
-        const float Jr[4] = {diff0 + diff1 * fri[0], diff0 - diff1 * fri[0], diff0 + diff2 * fri[1],
-                             diff0 - diff2 * fri[1]};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          d.efc_J[size_t(r + e) * nv + i] = Jr[e];
-          jq[e] += Jr[e] * qvel[i];
-        }
+    const bool trees = nv > 32;  // rows zeroed first, then written over the bodies' trees
+    if (trees) {
+      float* J = d.efc_J + size_t(adr + nlim) * nv;
+      const size_t cnt = size_t(4 * ncact) * nv;
+      if ((nv & 3) == 0) {
+        for (size_t e = lane; e < cnt / 4; e += 32) reinterpret_cast<float4*>(J)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        for (size_t e = lane; e < cnt; e += 32) J[e] = 0.f;
       }
-#pragma unroll
-      for (int e = 0; e < 4; e++) jq[e] = warp_sum(jq[e]);
-      if (lane < 4) {
-        const float fri0 = fri[0];
-        float invweight = m.body_invweight0[2 * b1] + m.body_invweight0[2 * b2];
+      __syncwarp();
+    }
+    // nv <= 32: the lane's dof is the same for every contact
+    s6 cd0{};
+    int db0 = 0;
+    float qv0 = 0.f;
+    if (!trees && lane < nv) {
+      cd0 = ld6(cdof + 6 * lane);
+      db0 = m.dof_bodyid[lane];
+      qv0 = qvel[lane];
+    }
+    int r = adr + nlim, held = 0;  // rows done, rows held by the lanes
+    int hc = 0, hb1 = 0, hb2 = 0;
+    float hpos = 0.f, hjq = 0.f;
+    auto flush = [&]() {
+      if (lane < held) {
+        const int row = r - held + lane;
+        const float fri0 = d.contact_friction[5 * hc];
+        float invweight = m.body_invweight0[2 * hb1] + m.body_invweight0[2 * hb2];
         invweight = invweight + fri0 * fri0 * invweight;
         invweight = invweight * 2.f * fri0 * fri0 / m.impratio;
-        const float jql = lane == 0 ? jq[0] : (lane == 1 ? jq[1] : (lane == 2 ? jq[2] : jq[3]));
-        d.efc_worldid[r + lane] = w;
-        update_efc_row(m, d, r + lane, pos, pos, invweight, d.contact_solref + 2 * c,
-                       d.contact_solimp + 5 * c, d.contact_includemargin[c], refsafe, jql);
+        d.efc_worldid[row] = w;
+        update_efc_row(m, d, row, hpos, hpos, invweight, d.contact_solref + 2 * hc,
+                       d.contact_solimp + 5 * hc, d.contact_includemargin[hc], refsafe, hjq);
       }
-      r += 4;
+      held = 0;
+    };
+    for (int base = 0; base < nc; base += 32) {
+      const int cl = ca + base + lane;
+      bool act = false;
+      float pos = 0.f, fr0 = 0.f, fr1 = 0.f, f[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      int b1 = 0, b2 = 0, a1 = 0, a2 = 0, z1 = 0, z2 = 0;
+      f3 off1{0.f, 0.f, 0.f}, off2{0.f, 0.f, 0.f};
+      if (base + lane < nc) {
+        const float dist = d.contact_dist[cl], margin = d.contact_includemargin[cl];
+        act = d.contact_dim[cl] == 3 && (dist - margin) < 0.f;
+        if (act) {
+          pos = dist - margin;
+          b1 = m.geom_bodyid[d.contact_geom[2 * cl]];
+          b2 = m.geom_bodyid[d.contact_geom[2 * cl + 1]];
+#pragma unroll
+          for (int e = 0; e < 9; e++) f[e] = d.contact_frame[9 * cl + e];
+          fr0 = d.contact_friction[5 * cl];
+          fr1 = d.contact_friction[5 * cl + 1];
+          const f3 cp = ld3(d.contact_pos + 3 * cl);
+          const int r1 = m.body_rootid[b1], r2 = m.body_rootid[b2];
+          off1 = cp - ld3(sc + 3 * r1);
+          off2 = cp - ld3(sc + 3 * r2);
+          if (trees) {
+            root_dofs(m, r1, a1, z1);
+            root_dofs(m, r2, a2, z2);
+          }
+        }
+      }
+      for (unsigned mask = __ballot_sync(WARP_FULL, act); mask; mask &= mask - 1u) {
+        const int src = __ffs(mask) - 1;
+        auto get = [&](auto v) { return __shfl_sync(WARP_FULL, v, src); };
+        const int c = ca + base + src, B1 = get(b1), B2 = get(b2);
+        const float P = get(pos);
+        const f3 O1{get(off1.x), get(off1.y), get(off1.z)}, O2{get(off2.x), get(off2.y), get(off2.z)};
+        const float fr[9] = {get(f[0]), get(f[1]), get(f[2]), get(f[3]), get(f[4]),
+                             get(f[5]), get(f[6]), get(f[7]), get(f[8])};
+        const float fri[2] = {get(fr0), get(fr1)};
+        float jq[4] = {0.f, 0.f, 0.f, 0.f};
+        auto dof = [&](int i, const s6& cd, int db, float qv) {
+          const f3 ang{cd.v[0], cd.v[1], cd.v[2]}, lin{cd.v[3], cd.v[4], cd.v[5]};
+          // constraint.py:76-101: the dof moves body b iff its body is an ancestor-or-self of b
+          const float in1 = (db != 0 && db <= B1 && B1 < m.body_subtreeend[db]) ? 1.f : 0.f;
+          const float in2 = (db != 0 && db <= B2 && B2 < m.body_subtreeend[db]) ? 1.f : 0.f;
+          const f3 j1 = (lin + cross(ang, O1)) * in1;
+          const f3 j2 = (lin + cross(ang, O2)) * in2;
+          const f3 jd = j2 - j1;
+          const float diff0 = fr[0] * jd.x + fr[1] * jd.y + fr[2] * jd.z;
+          const float diff1 = fr[3] * jd.x + fr[4] * jd.y + fr[5] * jd.z;
+          const float diff2 = fr[6] * jd.x + fr[7] * jd.y + fr[8] * jd.z;
+          const float Jr[4] = {diff0 + diff1 * fri[0], diff0 - diff1 * fri[0], diff0 + diff2 * fri[1],
+                               diff0 - diff2 * fri[1]};
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            d.efc_J[size_t(r + e) * nv + i] = Jr[e];
+            jq[e] += Jr[e] * qv;
+          }
+        };
+        if (trees) {  // the dofs of the two bodies' trees, each by its lane of the whole row
+          int lo = get(a1), lz = get(z1), ho = get(a2), hz = get(z2);
+          if (ho < lo) {
+            const int t = lo, tz = lz;
+            lo = ho, lz = hz, ho = t, hz = tz;
+          }
+          if (lo == ho) lz = lo = 0, hz = max(get(z1), get(z2));  // one tree (or one body without dofs)
+#pragma unroll 1
+          for (int q = 0; q < 2; q++) {
+            const int a = q ? ho : lo, z = q ? hz : lz;
+            for (int i = a + ((lane - a) & 31); i < z; i += 32)
+              dof(i, ld6(cdof + 6 * i), m.dof_bodyid[i], qvel[i]);
+          }
+        } else if (lane < nv) {
+          dof(lane, cd0, db0, qv0);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) jq[e] = warp_sum(jq[e]);
+        if ((lane >> 2) == (held >> 2)) {
+          const int e = lane & 3;
+          hc = c;
+          hb1 = B1;
+          hb2 = B2;
+          hpos = P;
+          hjq = e == 0 ? jq[0] : (e == 1 ? jq[1] : (e == 2 ? jq[2] : jq[3]));
+        }
+        held += 4;
+        r += 4;
+        if (held == 32) flush();
+      }
     }
+    flush();
   }
   __syncwarp();
 }

@@ -67,3 +67,62 @@ def test_small_solver_rows_per_world(nbox):
     c, best = cost(qacc[w]), cost(a)
     tol = (n[w] + mjm.nv) * 2.0 ** -24 * 10 * best + mjm.opt.tolerance * mjm.stat.meaninertia * mjm.nv * 10
     assert c <= best + max(tol, 1e-4 * best), (w, n[w], c, best)
+
+
+@pytest.mark.parametrize("model", ["humanoid", "humanoid_spheres", "bin"])
+def test_constraint_rows_vs_oracle(model):
+  """Rows of 1 to 50 contacts per world (scalars formed eight contacts at a time; past 32 dofs only the
+  dofs of the two bodies' trees are visited)."""
+  if model == "humanoid":
+    mjm = humanoid()
+    q, v, u = humanoid_state(mjm, 16, seed=5)
+  elif model == "bin":
+    mjm = load("bin.xml", jacobian=MJ_JAC_DENSE)
+    q, v, u = bin_state(mjm, 6, seed=9)
+  else:
+    mjm = load("humanoid_spheres.xml", jacobian=MJ_JAC_DENSE)
+    q, v, u, _ = humanoid_spheres_state(mjm, load("humanoid.xml"), 16, seed=9)
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, u, nconmax=600 * nworld, njmax=512 * nworld)
+  mjw.forward(m, d)
+  o = oracle(mjm, q, v, u, 32)
+  o.run("forward_nosolve")
+  torch.cuda.synchronize()
+  n, idx = world_rows(d, "efc")
+  cnt, D = o.rows("efc_D")
+  np.testing.assert_array_equal(n, cnt)
+  for name, t in (("efc_D", d.efc.D), ("efc_aref", d.efc.aref)):
+    got = t.cpu().numpy().astype(np.float64)[idx]
+    ref = np.asarray(o.rows(name)[1], dtype=np.float64).reshape(-1)
+    # the reference tests' tolerance on constraint rows
+    np.testing.assert_allclose(got, ref, rtol=2e-3, atol=2e-3 * max(1.0, np.abs(ref).max() * 1e-3), err_msg=name)
+  # J from the device's own contacts and motion axes in FP64 (the frame of two nearly parallel capsules
+  # depends on the last bits of their poses), within the roundings of a term of a row
+  cn, cidx = world_rows(d, "contact")
+  c = {k: getattr(d.contact, k).cpu().numpy()[cidx] for k in ("dist", "pos", "frame", "includemargin", "friction", "geom", "dim")}
+  J = d.efc.J.cpu().numpy().astype(np.float64)[idx]
+  cdof, com = dev(d.cdof).reshape(nworld, mjm.nv, 6), dev(d.subtree_com).reshape(nworld, mjm.nbody, 3)
+  gb, root, par = (np.asarray(x) for x in (mjm.geom_bodyid, mjm.body_rootid, mjm.body_parentid))
+  db = np.asarray(mjm.dof_bodyid)
+  chain = np.zeros((mjm.nbody, mjm.nv), dtype=bool)
+  for b in range(1, mjm.nbody):
+    chain[b] = chain[par[b]] | (db == b)
+  row = at = 0
+  for w in range(nworld):
+    act = [k for k in range(at, at + cn[w]) if c["dim"][k] == 3 and c["dist"][k] < c["includemargin"][k]]
+    at += cn[w]
+    row += n[w] - 4 * len(act)  # the limit rows
+    for k in act:
+      jac = []
+      for g in c["geom"][k]:
+        off = c["pos"][k].astype(np.float64) - com[w, root[gb[g]]]
+        jac.append((cdof[w, :, 3:] + np.cross(cdof[w, :, :3], off)) * chain[gb[g]][:, None])
+      diff = (jac[1] - jac[0]) @ c["frame"][k].astype(np.float64).reshape(3, 3).T
+      f = c["friction"][k]
+      for e, ref in enumerate((diff[:, 0] + f[0] * diff[:, 1], diff[:, 0] - f[0] * diff[:, 1],
+                               diff[:, 0] + f[1] * diff[:, 2], diff[:, 0] - f[1] * diff[:, 2])):
+        scale = max(1.0, np.abs(jac[0]).max(), np.abs(jac[1]).max())
+        assert np.abs(J[row + e] - ref).max() <= 32 * 2.0 ** -24 * scale * 4, (w, k, e)
+      row += 4
+  assert row == len(idx)
