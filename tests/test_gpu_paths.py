@@ -126,3 +126,44 @@ def test_constraint_rows_vs_oracle(model):
         assert np.abs(J[row + e] - ref).max() <= 32 * 2.0 ** -24 * scale * 4, (w, k, e)
       row += 4
   assert row == len(idx)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_step_io_copies_by_alignment(offset):
+  """Inputs and outputs at 4-byte offsets from 16-byte alignment give what aligned ones give."""
+  mjm = humanoid()
+  q, v, u = humanoid_state(mjm, 7, seed=4)
+  m = mjw.put_model(mjm)
+  outs = []
+  for off in (0, offset):
+    d = device_data(mjm, q, v, u)
+
+    def at(shape, src=None):
+      n = int(np.prod(shape))
+      t = torch.full((n + off + 4,), 7.0, device="cuda")
+      view = t[off:off + n].view(shape)
+      if src is not None:
+        view.copy_(torch.as_tensor(src, dtype=torch.float32))
+      return view
+
+    ins = {"qpos": at(q.shape, q), "qvel": at(v.shape, v), "ctrl": at(u.shape, u)}
+    out = {"qpos": at(q.shape), "qvel": at(v.shape), "xpos": at((7, mjm.nbody, 3))}
+    mjw.step_io(m, d, 2, inputs=ins, outputs=tuple(out), out=out)
+    torch.cuda.synchronize()
+    outs.append({k: t.clone() for k, t in out.items()})
+  for k in outs[0]:
+    assert torch.equal(outs[0][k], outs[1][k]), k
+
+
+def test_step_io_overlapping_buffers_keep_their_order():
+  """A copy whose source is another copy's destination: qvel comes from the Data's own warmstart,
+  which the next input then replaces."""
+  mjm = humanoid()
+  q, v, u = humanoid_state(mjm, 5, seed=2)
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, u, warmstart=v)
+  want = device_data(mjm, q, v, u)
+  mjw.step_io(m, d, 1, inputs={"qvel": d.qacc_warmstart, "qacc_warmstart": torch.zeros_like(d.qvel)}, outputs=())
+  mjw.step_io(m, want, 1, outputs=())
+  torch.cuda.synchronize()
+  assert torch.equal(d.qvel, want.qvel)
