@@ -770,57 +770,6 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
   return true;
 }
 
-// chol_tile on a tile whose rows fall into groups that do not couple (g: the mask of this lane's
-// group, 0 for lanes past the last row): every group takes its own four-column steps, so the tile
-// takes as many steps as its largest group instead of n / 4.  The columns outside a row's group are
-// zero, so each sum is chol_tile's.
-__device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned g, int lane) {
-  float* Ar = A + min(lane, n - 1) * ld;
-  unsigned cm = 0u;  // four-column chunks with columns of the group
-#pragma unroll
-  for (int j = 0; j < 8; j++)
-    if ((g >> (4 * j)) & 15u) cm |= 1u << j;
-  const unsigned all = cm;
-#pragma unroll 1
-  while (__any_sync(WARP_FULL, cm != 0u)) {
-    const int c = cm ? __ffs(cm) - 1 : 0, k = 4 * c;
-    const unsigned on = cm ? (g >> k) & 15u : 0u;
-    const float* Ak[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) Ak[j] = ((on >> j) & 1u) ? A + (k + j) * ld : Ar;
-    float s[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-#pragma unroll 1
-    for (unsigned pm = cm ? all & ((1u << c) - 1u) : 0u; pm; pm &= pm - 1u) {
-      const int q = 4 * (__ffs(pm) - 1);
-      const float4 a = *reinterpret_cast<const float4*>(Ar + q);
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float4 b = *reinterpret_cast<const float4*>(Ak[j] + q);
-        s[j][0] += a.x * b.x;
-        s[j][1] += a.y * b.y;
-        s[j][2] += a.z * b.z;
-        s[j][3] += a.w * b.w;
-      }
-    }
-    float l[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-#pragma unroll
-      for (int t = 0; t < j; t++) s[j][0] += l[t] * __shfl_sync(WARP_FULL, l[t], k + j);
-      const float x = Ar[k + j] - ((s[j][0] + s[j][1]) + (s[j][2] + s[j][3]));
-      const float piv = __shfl_sync(WARP_FULL, x, k + j);
-      if (((on >> j) & 1u) && lane >= k + j) {
-        l[j] = x * rsqrtf(piv);
-        Ar[k + j] = l[j];
-      }
-    }
-    __syncwarp();
-    cm &= cm - 1u;
-  }
-}
-
 // chol_cta over the nonzero tiles of S, on S.L: the same panels, products and sums.
 // (i) panel updates: a warp per two 8-row groups of trees t and one 8-column group of a panel's tree
 // u, over the 8-column chunks that hold a tree both couple with (rows and columns of an mma tile are

@@ -43,6 +43,17 @@ __device__ __forceinline__ void lsync() {
   else __syncwarp(((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)));
 }
 
+// zeros into p[0 .. n) by L lanes, 16 bytes a lane where p allows it
+template <int L>
+__device__ __forceinline__ void zero_fill(float* p, int n, int lane) {
+  int e = 0;
+  if ((reinterpret_cast<size_t>(p) & 15) == 0) {
+    e = n & ~3;
+    for (int i = lane; i < n / 4; i += L) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (e += lane; e < n; e += L) p[e] = 0.f;
+}
+
 // ------------------------------------------------------------------------------------------
 // smooth.py:32-145 — forward kinematics
 template <int L = 32>
@@ -351,7 +362,7 @@ __device__ void crb(const MjbModel& m, const MjbData& d, int w, int lane) {
   }
   // qM_dense (smooth.py:281-302)
   float* qM = d.qM + W(w, nv * nv);
-  for (int e = lane; e < nv * nv; e += L) qM[e] = 0.f;
+  zero_fill<L>(qM, nv * nv, lane);
   lsync<L>();
   for (int i = lane; i < nv; i += L) {
     const s6 ci = ld6(cdof + 6 * i);
@@ -569,6 +580,57 @@ __device__ MJB_TILE_FN void chol_tile(float* A, int ld, int n, int lane) {
   }
 }
 
+// chol_tile on a tile whose rows fall into groups that do not couple (g: the mask of this lane's
+// group, 0 for lanes past the last row): every group takes its own four-column steps, so the tile
+// takes as many steps as its largest group instead of n / 4.  The columns outside a row's group are
+// zero, so each sum is chol_tile's.
+__device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned g, int lane) {
+  float* Ar = A + min(lane, n - 1) * ld;
+  unsigned cm = 0u;  // four-column chunks with columns of the group
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    if ((g >> (4 * j)) & 15u) cm |= 1u << j;
+  const unsigned all = cm;
+#pragma unroll 1
+  while (__any_sync(WARP_FULL, cm != 0u)) {
+    const int c = cm ? __ffs(cm) - 1 : 0, k = 4 * c;
+    const unsigned on = cm ? (g >> k) & 15u : 0u;
+    const float* Ak[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) Ak[j] = ((on >> j) & 1u) ? A + (k + j) * ld : Ar;
+    float s[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll 1
+    for (unsigned pm = cm ? all & ((1u << c) - 1u) : 0u; pm; pm &= pm - 1u) {
+      const int q = 4 * (__ffs(pm) - 1);
+      const float4 a = *reinterpret_cast<const float4*>(Ar + q);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float4 b = *reinterpret_cast<const float4*>(Ak[j] + q);
+        s[j][0] += a.x * b.x;
+        s[j][1] += a.y * b.y;
+        s[j][2] += a.z * b.z;
+        s[j][3] += a.w * b.w;
+      }
+    }
+    float l[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+#pragma unroll
+      for (int t = 0; t < j; t++) s[j][0] += l[t] * __shfl_sync(WARP_FULL, l[t], k + j);
+      const float x = Ar[k + j] - ((s[j][0] + s[j][1]) + (s[j][2] + s[j][3]));
+      const float piv = __shfl_sync(WARP_FULL, x, k + j);
+      if (((on >> j) & 1u) && lane >= k + j) {
+        l[j] = x * rsqrtf(piv);
+        Ar[k + j] = l[j];
+      }
+    }
+    __syncwarp();
+    cm &= cm - 1u;
+  }
+}
+
 // x = (L L^T)^-1 y for an n <= 32 tile factor; lane i holds y_i and returns x_i (the arithmetic of
 // cho_solve32).  The forward pass reads the lane's own row four columns at a time, the backward
 // pass row k across the lanes; neither load depends on the substitution chain.
@@ -662,6 +724,111 @@ __device__ __noinline__ double cho_solve_tile_d(const double* L, int ld, int n, 
   }
   return own ? x : 0.0;
 }
+// chol_tile_d group by group, as chol_tile_groups
+__device__ __noinline__ void chol_tile_d_groups(double* A, int ld, int n, unsigned g, int lane) {
+  double* Ar = A + min(lane, n - 1) * ld;
+  unsigned cm = 0u;
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    if ((g >> (4 * j)) & 15u) cm |= 1u << j;
+  const unsigned all = cm;
+#pragma unroll 1
+  while (__any_sync(WARP_FULL, cm != 0u)) {
+    const int c = cm ? __ffs(cm) - 1 : 0, k = 4 * c;
+    const unsigned on = cm ? (g >> k) & 15u : 0u;
+    const double* Ak[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) Ak[j] = ((on >> j) & 1u) ? A + (k + j) * ld : Ar;
+    double s[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = 0.0;
+#pragma unroll 1
+    for (unsigned pm = cm ? all & ((1u << c) - 1u) : 0u; pm; pm &= pm - 1u) {
+      const int q = 4 * (__ffs(pm) - 1);
+#pragma unroll
+      for (int m = q; m < q + 4; m += 2) {
+        const double a0 = Ar[m], a1 = Ar[m + 1];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          s[j][0] += a0 * Ak[j][m];
+          s[j][1] += a1 * Ak[j][m + 1];
+        }
+      }
+    }
+    double l[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const double l0 = __shfl_sync(WARP_FULL, l[0], k + j), l1 = __shfl_sync(WARP_FULL, l[1], k + j),
+                   l2 = __shfl_sync(WARP_FULL, l[2], k + j);
+      if (j >= 1) s[j][0] += l[0] * l0;
+      if (j >= 2) s[j][1] += l[1] * l1;
+      if (j >= 3) s[j][0] += l[2] * l2;
+      const double x = Ar[k + j] - (s[j][0] + s[j][1]);
+      const double piv = __shfl_sync(WARP_FULL, x, k + j);
+      if (((on >> j) & 1u) && lane >= k + j) {
+        l[j] = x * rsqrt(piv);
+        Ar[k + j] = l[j];
+      }
+    }
+    __syncwarp();
+    cm &= cm - 1u;
+  }
+}
+// Four consecutive tree blocks of up to 8 dofs are factored and solved at once, block q in rows and
+// columns 8 q .. 8 q + 7 of the tile (its lanes: the octet q).  A block's four-column steps start at
+// its own first column in either place, so the factor is that of the block by itself.  One block at
+// a time left the warp waiting out 64 short chains per world of the bin (384 dofs) and 17 of the
+// humanoid with spheres.
+struct BlockPack {
+  int cnt;         // blocks, 0 or 1: not packed
+  int a, n;        // this lane's block: first dof and size (0: none)
+  unsigned group;  // its dofs in the tile, on the lanes that have one
+};
+__device__ __forceinline__ BlockPack pack_blocks(const MjbModel& m, int blk, int lane) {
+  const int b = blk + (lane >> 3);
+  const int n = b < m.nblock ? m.block_size[b] : 9;
+  const unsigned small = __ballot_sync(WARP_FULL, n <= 8);
+  BlockPack p;
+  p.cnt = (small & 0xffu) != 0xffu ? 0 : ((small & 0xffffu) != 0xffffu ? 1 : ((small & 0xffffffu) != 0xffffffu ? 2 : (small != WARP_FULL ? 3 : 4)));
+  const bool has = (lane >> 3) < p.cnt;
+  p.a = has ? m.block_adr[b] : 0;
+  p.n = has ? n : 0;
+  p.group = (lane & 7) < p.n ? ((1u << p.n) - 1u) << (lane & 24) : 0u;
+  return p;
+}
+// The pack's blocks of M (row stride ld) into the tile, zero between the blocks, 1 on the diagonal of
+// the rows that no block has.
+template <typename T>
+__device__ __forceinline__ void pack_load(const float* M, int ld, const BlockPack& p, T* tile, int tld, int lane) {
+  const int c = lane & 7, q = lane >> 3;
+  float v[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) v[r] = r < p.n && c < p.n ? M[size_t(p.a + r) * ld + p.a + c] : (r == c ? 1.f : 0.f);
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) tile[(8 * b + r) * tld + lane] = b == q ? T(v[r]) : T(0);
+}
+// cho_solve_tile of the pack's blocks: lane's row lr[j], j < c, and column lc[j], j > c, of its block
+template <typename T>
+__device__ __forceinline__ T pack_solve(const T (&lr)[8], const T (&lc)[8], T invd, T y, const BlockPack& p, int lane) {
+  const int c = lane & 7;
+  T z = c < p.n ? y : T(0);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    if (c == j) z *= invd;
+    const T zj = __shfl_sync(WARP_FULL, z, (lane & 24) + j);
+    if (c > j && c < p.n) z -= lr[j] * zj;
+  }
+#pragma unroll
+  for (int j = 7; j >= 0; j--) {
+    if (c == j) z *= invd;
+    const T zj = __shfl_sync(WARP_FULL, z, (lane & 24) + j);
+    if (c < j && j < p.n) z -= lc[j] * zj;
+  }
+  return z;
+}
+
 // Floats of per-warp scratch the precision form adds for its double tile.
 __host__ __device__ __forceinline__ int prec_tile_floats(int nv) { return 2 * tile_floats(nv); }
 
@@ -807,10 +974,31 @@ __device__ void factor_blocks(const MjbModel& m, const float* M, float* L, int l
   const int nv = m.nv;
   // one tiled block covering every dof is written whole by tile_store_lower
   if (!(tile && m.nblock == 1 && nv <= 32)) {
-    for (int e = lane; e < nv * nv; e += 32) L[e] = 0.f;
+    zero_fill<32>(L, nv * nv, lane);
     __syncwarp();
   }
   for (int blk = 0; blk < m.nblock; blk++) {
+    if (tile && nv >= 32) {  // a tile of 32 rows
+      const BlockPack p = pack_blocks(m, blk, lane);
+      if (p.cnt > 1) {
+        const int tld = tile_ld(nv), c = lane & 7, at = (lane & 24) * tld + lane;
+        pack_load(M, nv, p, tile, tld, lane);
+        __syncwarp();
+        if (dadd && c < p.n) {
+          float v = tile[at + c * tld];
+          v += scale * dadd[p.a + c];
+          tile[at + c * tld] = v;
+        }
+        __syncwarp();
+        chol_tile_groups(tile, tld, 32, p.group, lane);
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+          if (r < p.n && c < p.n) L[size_t(p.a + r) * nv + p.a + c] = c <= r ? tile[at + r * tld] : 0.f;
+        __syncwarp();
+        blk += p.cnt - 1;
+        continue;
+      }
+    }
     const int a = m.block_adr[blk], n = m.block_size[blk];
     if (tile && n <= 32) {
       const int tld = tile_ld(nv);
@@ -850,6 +1038,25 @@ __device__ void solve_blocks(const MjbModel& m, const float* L, float* x, const 
                              int lane, float* tile = nullptr, bool tile_has_factor = false) {
   const int nv = m.nv;
   for (int blk = 0; blk < m.nblock; blk++) {
+    if (m.nblock > 1) {
+      const BlockPack p = pack_blocks(m, blk, lane);
+      if (p.cnt > 1) {
+        const int c = lane & 7;
+        const float* Lb = L + size_t(p.a) * nv + p.a;
+        float lr[8], lc[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          lr[j] = j < c && c < p.n ? Lb[size_t(c) * nv + j] : 0.f;
+          lc[j] = j > c && j < p.n ? Lb[size_t(j) * nv + c] : 0.f;
+        }
+        const float invd = c < p.n ? __frcp_rn(Lb[size_t(c) * nv + c]) : 0.f;
+        const float xi = pack_solve(lr, lc, invd, c < p.n ? y[p.a + c] : 0.f, p, lane);
+        if (c < p.n) x[p.a + c] = xi;
+        __syncwarp();
+        blk += p.cnt - 1;
+        continue;
+      }
+    }
     const int a = m.block_adr[blk], n = m.block_size[blk];
     if (n <= 32) {
       const float yi = lane < n ? y[a + lane] : 0.f;
@@ -881,6 +1088,30 @@ __device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, const f
                                       float scale, float* x, const float* y, int lane, double* dt) {
   const int nv = m.nv, ld = tile_ld(nv);
   for (int blk = 0; blk < m.nblock; blk++) {
+    if (nv >= 32) {
+      const BlockPack p = pack_blocks(m, blk, lane);
+      if (p.cnt > 1) {
+        const int c = lane & 7, at = (lane & 24) * ld + lane;
+        pack_load(M, nv, p, dt, ld, lane);
+        __syncwarp();
+        if (dadd && c < p.n) dt[at + c * ld] += double(scale) * double(dadd[p.a + c]);
+        __syncwarp();
+        chol_tile_d_groups(dt, ld, 32, p.group, lane);
+        double lr[8], lc[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          lr[j] = j < c && c < p.n ? dt[lane * ld + (lane & 24) + j] : 0.0;
+          lc[j] = j > c && j < p.n ? dt[at + j * ld] : 0.0;
+        }
+        const double invd = c < p.n ? 1.0 / dt[at + c * ld] : 0.0;
+        const double xi = pack_solve(lr, lc, invd, c < p.n ? double(y[p.a + c]) : 0.0, p, lane);
+        __syncwarp();
+        if (c < p.n) x[p.a + c] = float(xi);
+        __syncwarp();
+        blk += p.cnt - 1;
+        continue;
+      }
+    }
     const int a = m.block_adr[blk], n = m.block_size[blk];
     for (int r = 0; r < n; r++)
       if (lane < n) {

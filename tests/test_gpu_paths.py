@@ -69,6 +69,59 @@ def test_small_solver_rows_per_world(nbox):
     assert c <= best + max(tol, 1e-4 * best), (w, n[w], c, best)
 
 
+def spheres_xml(sizes):
+  """Trees of the given numbers of slide / hinge dofs (6: a free sphere)."""
+  out = []
+  for i, s in enumerate(sizes):
+    if s == 6:
+      out.append(f'<body pos="{i} 0 1"><freejoint/><geom type="sphere" size="0.1"/></body>')
+      continue
+    chain, close = "", ""
+    for k in range(s):
+      chain += (f'<body pos="{i if k == 0 else 0} 0 {1 if k == 0 else -0.1}"><joint type="hinge" damping="0.3" axis="{k % 2} {(k + 1) % 2} 0.2"/>'
+                '<geom type="capsule" fromto="0 0 0 0.02 0 -0.1" size="0.02"/>')
+      close += "</body>"
+    out.append(chain + close)
+  return ('<mujoco><option timestep="0.002"><flag contact="disable"/></option><worldbody>' + "".join(out)
+          + "</worldbody></mujoco>")
+
+
+@pytest.mark.parametrize("form", [1, 3])
+@pytest.mark.parametrize("sizes", [(1, 8), (6, 5), (8, 9, 8, 8), (6,) * 6, (8, 1, 7, 6, 2, 27, 6, 6), (33, 6, 6)])
+def test_packed_tree_blocks(sizes, form):
+  """Factor, solve and damped integration of dense mass matrices of trees of 1 to 33 dofs: runs of
+  trees of up to 8 are taken four at a time (nv >= 32 for the factor).  L L' = M within the backward
+  error of an FP32 Cholesky factorisation of the largest block; qacc_smooth and the Euler step with implicit damping against
+  FP64 solves of the same matrices, within cond(M) roundings."""
+  if form == 3 and max(sizes) > 32:
+    pytest.skip("the precision form takes trees of up to 32 dofs")
+  mjm = load(spheres_xml(sizes), jacobian=MJ_JAC_DENSE)
+  nworld, rng = 5, np.random.default_rng(len(sizes))
+  q = np.tile(mjm.qpos0, (nworld, 1))
+  hinge = np.asarray(mjm.jnt_type) == 3
+  q[:, np.asarray(mjm.jnt_qposadr)[hinge]] += rng.uniform(-0.5, 0.5, (nworld, int(hinge.sum())))
+  v = rng.normal(0.0, 0.2, (nworld, mjm.nv))
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, np.zeros((nworld, 0)), nconmax=8 * nworld, njmax=64 * nworld)
+  mjw.step(m, d, fused=form)
+  torch.cuda.synchronize()
+  nv, h = mjm.nv, mjm.opt.timestep
+  M = dev(d.qM).reshape(nworld, nv, nv)
+  L = dev(d.qLD).reshape(nworld, nv, nv)
+  f, a = dev(d.qfrc_smooth), dev(d.qacc_smooth)
+  damp = np.asarray(mjm.dof_damping)
+  for w in range(nworld):
+    eps = 2.0 ** -24
+    assert np.linalg.norm(L[w] @ L[w].T - M[w]) <= 2 * (max(sizes) + 1) * eps * np.linalg.norm(M[w])
+    ref = np.linalg.solve(M[w], f[w])
+    assert np.linalg.norm(a[w] - ref) <= 4 * max(sizes) * eps * np.linalg.cond(M[w]) * np.linalg.norm(ref)
+    Md = M[w] + h * np.diag(damp)
+    step = (dev(d.qvel)[w] - v[w].astype(np.float32)) / h
+    ref = np.linalg.solve(Md, f[w] + dev(d.qfrc_constraint)[w])
+    tol = 4 * max(sizes) * eps * np.linalg.cond(Md) * np.linalg.norm(ref) + 2 * eps * np.linalg.norm(v[w]) / h
+    assert np.linalg.norm(step - ref) <= tol, (w, np.linalg.norm(step - ref), tol)
+
+
 @pytest.mark.parametrize("model", ["humanoid", "humanoid_spheres", "bin"])
 def test_constraint_rows_vs_oracle(model):
   """Rows of 1 to 50 contacts per world (scalars formed eight contacts at a time; past 32 dofs only the
