@@ -11,6 +11,7 @@
 //    the Hessian factor while the active set is unchanged) and k_integrate (Euler / implicitfast
 //    and the finiteness check in one kernel);
 //  - single (MJB_FORM_SINGLE): every stage of a world inside one warp of one kernel.
+// The solvers, the single form and the adjoint are translation units of their own (mjb_launch.cuh).
 // No entry point allocates memory or synchronises the stream (except mjb_world_status, which
 // copies results to the host).
 #include <cuda_runtime.h>
@@ -20,23 +21,10 @@
 #include <mutex>
 
 #include "mjb_deriv.cuh"
+#include "mjb_launch.cuh"
 #include "mjb_solver.cuh"
-#include "mjb_solver_cta.cuh"
+#include "mjb_state.cuh"
 
-// minimum resident CTAs per SM requested for the solver kernels (caps registers per thread at
-// 65536 / (128 * MJB_MINB)); with the staged / unstaged solver paths compiled apart, 4 (128
-// registers) measured 2 % faster than 5 (96 registers, spilling) on the humanoid at 8192 worlds
-#ifndef MJB_MINB
-#define MJB_MINB 4
-#endif
-// the default for the chosen form's FP32 persistent solver (k_solve_queue<false, false, *>),
-// which is compiled for 4 and for 5 (MjbTune.solver_ctas_per_sm): on the humanoid at 8192 worlds
-// 5 CTAs per SM (96 registers, with spills) measured 0.256 against 0.241 ms early in a run and
-// 0.381 against 0.352 ms once the worlds lie on the floor; the plain form's solver and the
-// precision solver were slower at 5
-#ifndef MJB_MINB_QUEUE
-#define MJB_MINB_QUEUE 5
-#endif
 // minimum resident CTAs per SM of the other stage kernels and of the integrator (64 registers)
 #ifndef MJB_MINB_STAGE
 #define MJB_MINB_STAGE 8
@@ -58,34 +46,17 @@ enum Stage {
   S_SOLVE, S_EULER, S_IMPLICIT, S_QACC_SMOOTH_COPY, S_CHECK, S_SAP
 };
 
-constexpr int kDefaultWarps = 4;
 
 
 // Kernels take the Model / Data views by value as __grid_constant__ parameters: the stages receive
 // them by reference, and without the qualifier every thread would copy both structs (~1.6 KB)
 // into its local memory whenever a reference reaches a function that is not inlined.
 
-// NaN / Inf check of the integrated state (sets MJB_WS_NONFINITE)
-__device__ void check_finite(const MjbModel& m, const MjbData& d, int w, int lane) {
-  bool bad = false;
-  for (int i = lane; i < m.nq; i += 32) bad |= !isfinite(d.qpos[W(w, m.nq) + i]);
-  for (int i = lane; i < m.nv; i += 32) {
-    bad |= !isfinite(d.qvel[W(w, m.nv) + i]);
-    bad |= !isfinite(d.qacc[W(w, m.nv) + i]);
-  }
-  if (__any_sync(WARP_FULL, bad) && lane == 0 && d.world_status) atomicOr(d.world_status + w, MJB_WS_NONFINITE);
-}
-
-__device__ __forceinline__ void copy_qacc_smooth(const MjbModel& m, const MjbData& d, int w, int lane) {
-  for (int i = lane; i < m.nv; i += 32) d.qacc[W(w, m.nv) + i] = d.qacc_smooth[W(w, m.nv) + i];
-  __syncwarp();
-}
-
-// the solver needs up to 128 registers; make_constraint's lanes hold a contact each and need 80 (6
-// CTAs per SM: the fastest of 5, 6 and 8 on 8192 and on 32768 humanoid worlds, by 1 %); every other
-// stage is held to 64 for occupancy
+// make_constraint's lanes hold a contact each and need 80 registers (6 CTAs per SM: the fastest of
+// 5, 6 and 8 on 8192 and on 32768 humanoid worlds, by 1 %); every other stage is held to 64 for
+// occupancy
 template <int STAGE>
-__global__ void __launch_bounds__(128, STAGE == S_SOLVE ? MJB_MINB : (STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB_STAGE))
+__global__ void __launch_bounds__(128, STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB_STAGE)
     k_stage(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int smem_per_warp) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
@@ -108,7 +79,6 @@ __global__ void __launch_bounds__(128, STAGE == S_SOLVE ? MJB_MINB : (STAGE == S
     case S_SAP: sap_broadphase(m, d, w, lane, sm); break;
     case S_NARROW: primitive_narrowphase(m, d, w, lane); break;
     case S_MAKE_CONSTRAINT: make_constraint(m, d, w, lane); break;
-    case S_SOLVE: solve(m, d, w, lane, sm, d.efc_h + W(w, m.nv * m.nv)); break;
     case S_EULER: euler(m, d, w, lane, sm); break;
     case S_IMPLICIT: implicit(m, d, w, lane, sm); break;
     case S_QACC_SMOOTH_COPY: copy_qacc_smooth(m, d, w, lane); break;
@@ -134,51 +104,6 @@ __global__ void __launch_bounds__(128, MJB_MINB_STAGE)
     case S_FWD_VELOCITY: fwd_velocity<L>(m, d, w, lane); break;
     case S_FWD_ACTUATION: fwd_actuation<L>(m, d, w, lane); break;
   }
-}
-
-// whole forward (+ integration) of one world per warp; each warp's slice of dynamic shared memory
-// holds the solver's workspace, whose leading factor tile also serves the mass-matrix
-// factorisations (factor_m, then the integrator)
-__global__ void __launch_bounds__(128, MJB_MINB) k_step_fused(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int integrate,
-                                                    int smem_per_warp) {
-  extern __shared__ __align__(16) float smem[];
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  const int w = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (w >= d.nworld) return;
-  const int nv = m.nv;
-  float* sm = smem_per_warp ? smem + size_t(wib) * smem_per_warp : nullptr;
-  float* hs = d.efc_h + W(w, nv * nv);
-  kinematics(m, d, w, lane);
-  com_pos(m, d, w, lane);
-  crb(m, d, w, lane);
-  factor_m(m, d, w, lane, sm);
-  collision(m, d, w, lane, sm);
-  make_constraint(m, d, w, lane);
-  transmission(m, d, w, lane);
-  fwd_velocity(m, d, w, lane);
-  fwd_actuation(m, d, w, lane);
-  fwd_acceleration(m, d, w, lane, sm, true);  // the tile still holds factor_m's factor
-  if (d.njmax == 0) copy_qacc_smooth(m, d, w, lane);
-  else solve(m, d, w, lane, sm, hs, true);
-  if (integrate) {
-    if (m.integrator == 0) euler(m, d, w, lane, sm);
-    else implicit(m, d, w, lane, sm);
-    check_finite(m, d, w, lane);
-  }
-}
-
-// chosen form: the constraint solver with the Hessian factor kept across iterations; TC: the
-// Newton Hessian of up to 32 staged rows assembled on the tensor pipe in split TF32 (hessian_tc;
-// always in the precision form, an autotuner choice in the chosen form)
-template <bool PREC, bool TC>
-__global__ void __launch_bounds__(128, MJB_MINB) k_solve(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int smem_per_warp) {
-  extern __shared__ __align__(16) float smem[];
-  const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= d.nworld) return;
-  float* sm = smem_per_warp ? smem + size_t(threadIdx.x >> 5) * smem_per_warp : nullptr;
-  solve<PREC, TC>(m, d, w, lane, sm, d.efc_h + W(w, m.nv * m.nv), true);
 }
 
 // The chosen form's solver schedule.  k_order_worlds sorts the worlds by their constraint row
@@ -257,43 +182,6 @@ __global__ void __launch_bounds__(1024) k_order_worlds(const int* nefc, int* ord
   }
 }
 
-template <bool PREC, bool TC, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_solve_queue(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int smem_per_warp) {
-  extern __shared__ __align__(16) float smem[];
-  const int lane = threadIdx.x & 31;
-  float* sm = smem_per_warp ? smem + size_t(threadIdx.x >> 5) * smem_per_warp : nullptr;
-  for (;;) {
-    int idx = 0;
-    if (lane == 0) idx = atomicAdd(d.work_queue, 1);
-    idx = __shfl_sync(WARP_FULL, idx, 0);
-    if (idx >= d.nworld) break;
-    const int w = d.world_order[idx];
-    solve<PREC, TC>(m, d, w, lane, sm, d.efc_h + W(w, m.nv * m.nv), true);
-  }
-}
-
-// chosen form, models with nv > 32: one CTA of NW warps per world (mjb_solver_cta.cuh),
-// persistent over the work queue in k_order_worlds' order when the Data has the schedule arrays,
-// else one CTA per world in index order
-template <int NW, bool PREC>
-__global__ void __launch_bounds__(NW * 32, NW >= 16 ? 1 : (NW >= 8 ? 2 : (NW >= 4 ? 4 : (NW >= 2 ? 8 : 9))))
-    k_solve_cta(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int tc) {
-  extern __shared__ __align__(16) float smem[];
-  __shared__ int s_idx;
-  if (!d.work_queue) {
-    if (int(blockIdx.x) < d.nworld) solve_cta<NW, PREC>(m, d, blockIdx.x, smem, tc != 0);
-    return;
-  }
-  for (;;) {
-    if (threadIdx.x == 0) s_idx = atomicAdd(d.work_queue, 1);
-    __syncthreads();
-    const int idx = s_idx;
-    __syncthreads();
-    if (idx >= d.nworld) break;
-    solve_cta<NW, PREC>(m, d, d.world_order[idx], smem, tc != 0);
-  }
-}
-
 // chosen form: integration (forward.py:165-405) and the finiteness check
 __global__ void __launch_bounds__(128, MJB_MINB_INT) k_integrate(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int tile_per_warp) {
   extern __shared__ __align__(16) float smem[];
@@ -327,18 +215,6 @@ __global__ void k_fd_jacobian(const __grid_constant__ MjbModel m, const __grid_c
   if (t >= (long long)nworld * ncol) return;
   const int w = int(t / ncol), col = int(t - (long long)w * ncol);
   fd_column(m, p, w, col, flags, eps, A, B, lane);
-}
-// one warp per world; per_warp floats of dynamic shared memory per warp (step_vjp_floats)
-__global__ void __launch_bounds__(128) k_step_vjp(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d,
-                                                  const float* lam, const float* qvel_prev,
-                                                  float* grad_ctrl, float* grad_qvel,
-                                                  float* grad_qpos, int per_warp) {
-  extern __shared__ __align__(16) float smem[];
-  const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= d.nworld) return;
-  step_vjp_world(m, d, w, lane, lam, qvel_prev, grad_ctrl, grad_qvel, grad_qpos,
-                 smem + size_t(threadIdx.x >> 5) * per_warp);
 }
 // one warp per world
 __global__ void k_transition_vjp(const __grid_constant__ MjbModel m, int nworld, const float* A,
@@ -447,12 +323,7 @@ using namespace mjb;
 
 namespace {
 
-inline int grid_for(int nworld, int warps) { return (nworld + warps - 1) / warps; }
 
-inline int finish() {
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MJB_OK : MJB_ERR_LAUNCH;
-}
 
 // implicitfast needs the dense mass matrix (the reference asserts it, forward.py:268)
 inline bool implicit_unsupported(const MjbModel* m) { return m->is_sparse && m->integrator != 0; }
@@ -462,7 +333,7 @@ inline bool implicit_unsupported(const MjbModel* m) { return m->is_sparse && m->
 // CTA's shared memory (227 KB: nv up to about 230)
 int precision_supported(const MjbModel* m) {
   if (m->is_sparse || m->block_max > 32) return MJB_ERR_UNSUPPORTED;
-  if (m->nv > 32 && size_t(cta_solver_smem_floats(m->nv, 16, true)) * sizeof(float) > 227 * 1024)
+  if (m->nv > 32 && solver_cta_prec_smem(m->nv) > 227 * 1024)
     return MJB_ERR_SCRATCH;
   return MJB_OK;
 }
@@ -619,70 +490,28 @@ int fused_smem_per_warp(const MjbModel* m) {
   return m->ngeom > 100 ? std::max(spw, sap_smem_floats(m->ngeom)) : spw;
 }
 
-// dynamic shared memory a CTA of kDefaultWarps warps may use (the opt-in limit of sm_100)
-constexpr size_t kMaxSmemPerCta = 227 * 1024;
-
-// opts a kernel in to more than 48 KB of dynamic shared memory (once per kernel, device and size)
-constexpr int kSmemDevices = 64;
-template <typename K>
-void allow_smem(K kernel, size_t bytes, size_t (&configured)[kSmemDevices]) {
-  if (bytes <= 48 * 1024) return;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= kSmemDevices || bytes > configured[dev]) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    if (dev >= 0 && dev < kSmemDevices) configured[dev] = bytes;
-  }
-}
-
-// CTAs of `kernel` resident on the whole GPU at once for blocks of `threads` threads and `smem`
-// bytes, queried once per (device, kernel, block size, shared-memory size)
-template <typename K>
-int resident_ctas(K kernel, int threads, size_t smem) {
-  struct Entry {
-    int dev;
-    const void* fn;
-    int threads;
-    size_t smem;
-    int ctas;
-  };
-  static Entry cache[64];
-  static int used = 0;
-  static std::mutex mu;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const void* fn = reinterpret_cast<const void*>(kernel);
-  std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < used; i++)
-    if (cache[i].dev == dev && cache[i].fn == fn && cache[i].threads == threads &&
-        cache[i].smem == smem)
-      return cache[i].ctas;
-  int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  const int n = std::max(1, sms * std::max(1, per_sm));
-  if (used < 64) cache[used++] = Entry{dev, fn, threads, smem, n};
-  return n;
-}
 
 template <int STAGE>
 int launch_stage(const MjbModel* m, const MjbData* d, cudaStream_t s) {
   if (int rc = stage_fields(STAGE, m, d)) return rc;
-  const int warps = kDefaultWarps;
-  int spw = 0;
-  size_t bytes = 0;
-  if (STAGE == S_SOLVE) spw = m->nv <= 32 ? int(solver_smem_floats(m->nv)) : generic_nz_floats(m->nv);
-  if (STAGE == S_FACTOR_M || STAGE == S_FWD_ACCELERATION || STAGE == S_EULER || STAGE == S_IMPLICIT)
-    spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
-  if (STAGE == S_SAP) spw = sap_smem_floats(m->ngeom);
-  if (spw) {
-    bytes = size_t(spw) * warps * sizeof(float);
-    if (bytes > kMaxSmemPerCta) return MJB_ERR_SCRATCH;
-    static size_t configured[kSmemDevices];
-    allow_smem(k_stage<STAGE>, bytes, configured);
+  if constexpr (STAGE == S_SOLVE) {
+    return launch_solver_plain(m, d, s);
+  } else {
+    const int warps = kDefaultWarps;
+    int spw = 0;
+    size_t bytes = 0;
+    if (STAGE == S_FACTOR_M || STAGE == S_FWD_ACCELERATION || STAGE == S_EULER || STAGE == S_IMPLICIT)
+      spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
+    if (STAGE == S_SAP) spw = sap_smem_floats(m->ngeom);
+    if (spw) {
+      bytes = size_t(spw) * warps * sizeof(float);
+      if (bytes > kMaxSmemPerCta) return MJB_ERR_SCRATCH;
+      static size_t configured[kSmemDevices];
+      allow_smem(k_stage<STAGE>, bytes, configured);
+    }
+    k_stage<STAGE><<<grid_for(d->nworld, warps), 32 * warps, bytes, s>>>(*m, *d, spw);
+    return finish();
   }
-  k_stage<STAGE><<<grid_for(d->nworld, warps), 32 * warps, bytes, s>>>(*m, *d, spw);
-  return finish();
 }
 
 // the reference's broadphase choice (collision_driver.py:537-540)
@@ -714,7 +543,7 @@ struct ChosenCfg {
   int warps = kDefaultWarps;
   int cta_warps = 4;  // warps per world of the solver for nv > 32 (0: one warp per world)
   int hessian_tc = 0; // nv <= 32: Newton Hessian on the tensor pipe (split TF32) instead of FMAs
-  int solver_ctas = MJB_MINB_QUEUE;  // CTAs per SM of the FP32 FMA-Hessian persistent solver (4, 5)
+  int solver_ctas = 5;  // CTAs per SM of the FP32 FMA-Hessian persistent solver (4, 5)
 };
 struct TuneEntry {
   int dev, nv, cap;
@@ -858,59 +687,14 @@ int run_forward_plain(const MjbModel* m, const MjbData* d, cudaStream_t s) {
 
 // the chosen form's solver launch: k_order_worlds + the persistent k_solve_queue when the Data has
 // the schedule arrays, else one warp per world (k_solve); PREC selects the precision form's solver
-template <int NW, bool PREC>
-void launch_solver_cta(const MjbModel* m, const MjbData* d, int tc, cudaStream_t s) {
-  const size_t bytes = size_t(cta_solver_smem_floats(m->nv, NW, PREC)) * sizeof(float);
-  static size_t conf[kSmemDevices];
-  allow_smem(k_solve_cta<NW, PREC>, bytes, conf);
-  if (d->world_order && d->work_queue && d->world_nefc) {
-    const int ctas = resident_ctas(k_solve_cta<NW, PREC>, 32 * NW, bytes);  // ordered in phase 0
-    k_solve_cta<NW, PREC><<<std::min(ctas, d->nworld), 32 * NW, bytes, s>>>(*m, *d, tc);
-  } else {
-    MjbData dd = *d;
-    dd.work_queue = nullptr;
-    k_solve_cta<NW, PREC><<<d->nworld, 32 * NW, bytes, s>>>(*m, dd, tc);
-  }
-}
-
-template <bool PREC, bool TC, int MINB>
-void launch_solver_queue(const MjbModel* m, const MjbData* d, int qw, int spw, cudaStream_t s) {
-  const size_t qbytes = size_t(spw) * qw * sizeof(float);
-  static size_t conf_queue[kSmemDevices];
-  allow_smem(k_solve_queue<PREC, TC, MINB>, size_t(spw) * kDefaultWarps * sizeof(float), conf_queue);
-  const int ctas = resident_ctas(k_solve_queue<PREC, TC, MINB>, 32 * qw, qbytes);  // ordered in phase 0
-  k_solve_queue<PREC, TC, MINB><<<std::min(ctas, grid_for(d->nworld, qw)), 32 * qw, qbytes, s>>>(*m, *d, spw);
-}
-
-template <bool PREC, bool TC>
-void launch_solver_warp(const MjbModel* m, const MjbData* d, const ChosenCfg& cfg, int spw,
-                        cudaStream_t s) {
-  if (d->world_order && d->work_queue && d->world_nefc) {
-    if constexpr (PREC || TC) {
-      launch_solver_queue<PREC, TC, MJB_MINB>(m, d, cfg.warps, spw, s);
-    } else {
-      if (cfg.solver_ctas == 4) launch_solver_queue<PREC, TC, 4>(m, d, cfg.warps, spw, s);
-      else launch_solver_queue<PREC, TC, 5>(m, d, cfg.warps, spw, s);
-    }
-  } else {
-    const size_t bytes = size_t(spw) * kDefaultWarps * sizeof(float);
-    static size_t conf_solve[kSmemDevices];
-    allow_smem(k_solve<PREC, TC>, bytes, conf_solve);
-    k_solve<PREC, TC><<<grid_for(d->nworld, kDefaultWarps), 32 * kDefaultWarps, bytes, s>>>(*m, *d, spw);
-  }
-}
-
 template <bool PREC>
 void launch_solver(const MjbModel* m, const MjbData* d, const ChosenCfg& cfg, int spw,
                    cudaStream_t s) {
   // nv > 32: the CTA solver (the precision form's FP64 Hessian factor needs it)
   if (m->nv > 32 && (cfg.cta_warps > 0 || PREC)) {
-    const int tc = cfg.hessian_tc;
-    const int nw = cfg.cta_warps > 0 ? cfg.cta_warps : 4;  // the precision form's default: 4
-    if (nw == 2) launch_solver_cta<2, PREC>(m, d, tc, s);
-    else if (nw == 4) launch_solver_cta<4, PREC>(m, d, tc, s);
-    else if (nw == 16) launch_solver_cta<16, PREC>(m, d, tc, s);
-    else launch_solver_cta<8, PREC>(m, d, tc, s);
+    // the precision form's default: 4 warps per world
+    if (PREC) launch_solver_cta_prec(m, d, cfg.cta_warps > 0 ? cfg.cta_warps : 4, s);
+    else launch_solver_cta(m, d, cfg.cta_warps, cfg.hessian_tc, s);
     return;
   }
   // one warp per world on the nonzero trees and tiles (the generic solver's arithmetic, which takes
@@ -918,14 +702,14 @@ void launch_solver(const MjbModel* m, const MjbData* d, const ChosenCfg& cfg, in
   // iterations: solver 7.7 ms with the dense one-warp form, 2.2 ms so, step 8.27 -> 2.91 ms; one
   // tree has nothing to skip and stays with the dense form
   if constexpr (!PREC) {
-    if (m->nv > 32 && sparse_model<SparseFor<1>>(*m)) {
-      launch_solver_cta<1, false>(m, d, 0, s);
+    if (m->nv > 32 && solver_cta_takes_warp(m)) {
+      launch_solver_cta(m, d, 1, 0, s);
       return;
     }
   }
-  if (PREC) launch_solver_warp<PREC, true>(m, d, cfg, spw, s);
-  else if (cfg.hessian_tc) launch_solver_warp<PREC, true>(m, d, cfg, spw, s);
-  else launch_solver_warp<PREC, false>(m, d, cfg, spw, s);
+  if (PREC) launch_solver_warp_prec(m, d, cfg.warps, spw, s);
+  else if (cfg.hessian_tc || cfg.solver_ctas == 4) launch_solver_warp_alt(m, d, cfg.hessian_tc != 0, cfg.warps, spw, s);
+  else launch_solver_warp(m, d, cfg.warps, spw, s);
 }
 
 struct Copy {
@@ -1030,9 +814,7 @@ int run_fused(const MjbModel* m, const MjbData* d, const MjbRunCfg* cfg, int int
   const int spw = fused_smem_per_warp(m);
   const size_t smem = size_t(spw) * warps * sizeof(float);
   if (smem > kMaxSmemPerCta) return MJB_ERR_SCRATCH;
-  static size_t configured[kSmemDevices];
-  allow_smem(k_step_fused, smem, configured);
-  k_step_fused<<<grid_for(d->nworld, warps), 32 * warps, smem, s>>>(*m, *d, integrate, spw);
+  launch_step_fused(m, d, integrate, warps, spw, smem, s);
   return finish();
 }
 
@@ -1481,20 +1263,7 @@ static int launch_step_vjp(const MjbModel* m, const MjbData* d, const float* lam
   if (grad_qpos && (!d->rne_cacc || !d->rne_cfrc || !d->xanchor || !d->xaxis || !d->xipos ||
                     !d->ximat || !d->subtree_com || !d->qacc_integration))
     return MJB_ERR_ARG;
-  const int per_warp = (step_vjp_floats(*m, grad_qvel != nullptr, grad_qpos != nullptr) + 3) & ~3;
-  const size_t warp_bytes = size_t(per_warp) * sizeof(float);
-  int warps = 4;
-  while (warps > 1 && warps * warp_bytes > 48 * 1024) warps >>= 1;
-  const size_t bytes = warps * warp_bytes;
-  if (bytes > 227 * 1024) return MJB_ERR_SCRATCH;
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_step_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(bytes));
-    if (e != cudaSuccess) return MJB_ERR_LAUNCH;
-  }
-  k_step_vjp<<<grid_for(d->nworld, warps), 32 * warps, bytes, (cudaStream_t)stream>>>(
-      *m, *d, lam, qvel_prev, grad_ctrl, grad_qvel, grad_qpos, per_warp);
-  return finish();
+  return run_step_vjp(m, d, lam, qvel_prev, grad_ctrl, grad_qvel, grad_qpos, (cudaStream_t)stream);
 }
 
 extern "C" int mjb_ctrl_vjp(const MjbModel* m, const MjbData* d, const float* lam, float* grad_ctrl,

@@ -70,7 +70,7 @@ __device__ __forceinline__ f3 tan3(D3 a) { return mk3(a.x.d, a.y.d, a.z.d); }
 struct DFrame {
   D3 r[3];
 };
-__device__ DFrame dmake_frame(D3 a) {
+static __device__ DFrame dmake_frame(D3 a) {
   a = dnormalize(a);
   D3 b = (-0.5f < a.y.v && a.y.v < 0.5f) ? dc3(mk3(0.f, 1.f, 0.f)) : dc3(mk3(0.f, 0.f, 1.f));
   b = b - a * ddot(a, b);
@@ -78,13 +78,13 @@ __device__ DFrame dmake_frame(D3 a) {
   if (dlength(a).v == 0.f) b = dc3(mk3(0.f, 0.f, 0.f));
   return DFrame{{a, b, dcross(a, b)}};
 }
-__device__ D3 dclosest_segment_point(D3 a, D3 b, D3 pt) {
+static __device__ D3 dclosest_segment_point(D3 a, D3 b, D3 pt) {
   const D3 ab = b - a;
   Dl t = ddot(pt - a, ab) / (ddot(ab, ab) + dc(1e-6f));
   t = dclamp(t, 0.f, 1.f);
   return a + ab * t;
 }
-__device__ void dclosest_segment_to_segment_points(D3 a0, D3 a1, D3 b0, D3 b1, D3& pa, D3& pb) {
+static __device__ void dclosest_segment_to_segment_points(D3 a0, D3 a1, D3 b0, D3 b1, D3& pa, D3& pb) {
   const D3 da = a1 - a0, db = b1 - b0;
   const Dl la = dlength(da), lb = dlength(db);
   const D3 dir_a = la.v == 0.f ? da : da * (dc(1.f) / la);
@@ -131,7 +131,7 @@ __device__ __forceinline__ void dsphere_sphere(D3 p1, Dl r1, D3 p2, Dl r2, DCont
 
 // Candidate j of the narrowphase of one geom pair (narrow_pair's formulas and branches), the two
 // geom poses given as dual numbers.  Returns false when the pair has no candidate j.
-__device__ bool dcontact_candidate(const MjbModel& m, int g1, int g2, D3 p1, const D3* R1, D3 p2,
+static __device__ bool dcontact_candidate(const MjbModel& m, int g1, int g2, D3 p1, const D3* R1, D3 p2,
                                    const D3* R2, float margin, int j, DContact& c) {
   // R1 / R2: the columns of the geoms' rotation matrices
   const int t1 = m.geom_type[g1], t2 = m.geom_type[g2];
@@ -195,7 +195,7 @@ __device__ bool dcontact_candidate(const MjbModel& m, int g1, int g2, D3 p1, con
 // lane k < 12 differentiates along pose direction k (geom k / 6; translation for k % 6 < 3, else
 // rotation about world axis k % 3), the candidate whose position matches the stored contact is
 // taken, and the lane returns d(dist, pos, frame) / d(direction k) . bars.
-__device__ float contact_pose_bar(const MjbModel& m, const MjbData& d, int w, int c, float distb,
+static __device__ float contact_pose_bar(const MjbModel& m, const MjbData& d, int w, int c, float distb,
                                   f3 posb, const float* frameb, int lane) {
   const int g1 = d.contact_geom[2 * c], g2 = d.contact_geom[2 * c + 1];
   const float* gxpos = d.geom_xpos + W(w, 3 * m.ngeom);
@@ -242,7 +242,7 @@ __device__ float contact_pose_bar(const MjbModel& m, const MjbData& d, int w, in
 struct EfcPar {
   float k, b, imp, dimp;  // stiffness, damping, impedance, d imp / d pos
 };
-__device__ EfcPar efc_params(const MjbModel& m, const float* solref, const float* solimp, float pos,
+static __device__ EfcPar efc_params(const MjbModel& m, const float* solref, const float* solimp, float pos,
                              bool refsafe) {
   float timeconst = solref[0], dampratio = solref[1];
   float dmin = solimp[0], dmax = solimp[1], width = solimp[2], mid = solimp[3], power = solimp[4];
@@ -314,7 +314,7 @@ __device__ __forceinline__ void add6(float* p, const s6& a) {
 }
 
 // U_b = sum of u_i cdof_i over the dofs from the root to body b (a top-down sweep)
-__device__ void tree_sum_down(const MjbModel& m, const float* cdof, const float* u, float* U,
+static __device__ void tree_sum_down(const MjbModel& m, const float* cdof, const float* u, float* U,
                               int lane) {
   if (lane < 6) U[lane] = 0.f;
   __syncwarp();
@@ -331,7 +331,7 @@ __device__ void tree_sum_down(const MjbModel& m, const float* cdof, const float*
   }
 }
 // A_b += sum of A over b's children, deepest level first: subtree sums (body 0 untouched)
-__device__ void tree_sum_up(const MjbModel& m, float* A, int lane) {
+static __device__ void tree_sum_up(const MjbModel& m, float* A, int lane) {
   for (int lvl = m.nlevel - 1; lvl >= 1; lvl--) {
     const int beg = m.body_treeadr[lvl], end = m.body_treeadr[lvl + 1];
     for (int n = beg + lane; n < end; n += 32) {
@@ -348,7 +348,7 @@ __device__ void tree_sum_up(const MjbModel& m, float* A, int lane) {
 // Bars of u' M(q) x: with U_b, X_b the tree sums of u and x, u' M x = sum_b U_b . I_b X_b, so
 // cinert_b gets d(U_b' I X_b)/dc and cdof_i gets u_i (subtree sum of I X) + x_i (of I U).
 // Scratch: SA..SD, 6 nbody floats each.
-__device__ void mass_product_bars(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void mass_product_bars(const MjbModel& m, const MjbData& d, int w, int lane,
                                   const float* u, const float* x, float* cdof_bar, float* cinert_bar,
                                   float* SA, float* SB, float* SC, float* SD) {
   const int nb = m.nbody, nv = m.nv;
@@ -378,7 +378,7 @@ __device__ void mass_product_bars(const MjbModel& m, const MjbData& d, int w, in
 
 // Bars of u' qfrc_bias(q, v) on cdof and cinert (v = qv, the step's starting velocity): the
 // com_vel / rne recursions of the forward run backwards (see rne_vel_vjp for the velocity part).
-__device__ void bias_q_bars(const MjbModel& m, const MjbData& d, int w, int lane, const float* u,
+static __device__ void bias_q_bars(const MjbModel& m, const MjbData& d, int w, int lane, const float* u,
                             const float* qv, float* cdof_bar, float* cinert_bar, float* SA, float* SB,
                             float* SC) {
   const int nb = m.nbody, nv = m.nv;
@@ -461,7 +461,7 @@ __device__ void bias_q_bars(const MjbModel& m, const MjbData& d, int w, int lane
 // subtree_com[root(b)] kept in body b's slot).
 // With GV non-null the rows' velocity term -D_i b_i J_i (J_i s) of d loss / d qvel is subtracted
 // from GV (per dof) as well; with cdof_bar null only that is done.
-__device__ void row_q_bars(const MjbModel& m, const MjbData& d, int w, int lane, const float* S,
+static __device__ void row_q_bars(const MjbModel& m, const MjbData& d, int w, int lane, const float* S,
                            const float* qv, float* Q, float* cdof_bar, float* BF, float* BT,
                            float* SCB, float* GV) {
   const bool posq = cdof_bar != nullptr;
@@ -610,7 +610,7 @@ __device__ void row_q_bars(const MjbModel& m, const MjbData& d, int w, int lane,
 // joint) and torques of the body frames whose columns free / ball cdof use (BT).  com_pos: a hinge
 // has cdof = (axis; axis x off), a slide (0; axis), a free / ball rotational dof (x_k; x_k x off)
 // with x_k the body frame's column k, off = subtree_com[root] - anchor.
-__device__ void cdof_joint_bars(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void cdof_joint_bars(const MjbModel& m, const MjbData& d, int w, int lane,
                                 const float* cdof_bar, float* JA, float* JX, float* JS, float* BT) {
   const float* xmat = d.xmat + W(w, 9 * m.nbody);
   const float* xanchor = d.xanchor + W(w, 3 * m.njnt);
@@ -651,7 +651,7 @@ __device__ void cdof_joint_bars(const MjbModel& m, const MjbData& d, int w, int 
 
 // cinert bars -> body force / torque (xipos point, ximat columns) and SCB.  com_pos: cinert holds
 // R diag(inertia) R' (R = ximat) plus the parallel-axis terms of dif = xipos - subtree_com[root].
-__device__ void cinert_body_bars(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void cinert_body_bars(const MjbModel& m, const MjbData& d, int w, int lane,
                                  const float* cinert_bar, float* BF, float* BT, float* SCB) {
   const int nb = m.nbody;
   const float* xipos = d.xipos + W(w, 3 * nb);
@@ -692,7 +692,7 @@ __device__ void cinert_body_bars(const MjbModel& m, const MjbData& d, int w, int
 // subtree_com[r] = sum over r's subtree of mass_c xipos_c / subtree_mass_r: the bars collected
 // for each root r (SCB of its bodies, JS of its joints) become xipos forces on its bodies.
 // Scratch SR: 3 nbody floats.
-__device__ void subtree_com_bars(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void subtree_com_bars(const MjbModel& m, const MjbData& d, int w, int lane,
                                  const float* SCB, const float* JS, float* BF, float* BT, float* SR) {
   const int nb = m.nbody;
   const float* xipos = d.xipos + W(w, 3 * nb);
@@ -724,7 +724,7 @@ __device__ void subtree_com_bars(const MjbModel& m, const MjbData& d, int w, int
 // body, the descendant bodies), so with (F, T) summed over the downstream bars, a hinge gets
 // axis . (T - anchor x F), a slide axis . F, a free joint F (translation) and x_k . (T - pos x F)
 // (rotation about local axis k), a ball x_k . (T - anchor x F).  Adds to Q (per dof).
-__device__ void kinematic_sweep(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void kinematic_sweep(const MjbModel& m, const MjbData& d, int w, int lane,
                                 const float* JA, const float* JX, float* BF, float* BT, float* Q) {
   const int nb = m.nbody;
   const float* xpos = d.xpos + W(w, 3 * nb);

@@ -51,7 +51,7 @@ __device__ __forceinline__ int reserve(int* counter, int count, int cap, uint32_
 }
 
 // collision_driver.py:458-512 + _add_geom_pair (:52-68)
-__device__ void nxn_broadphase(const MjbModel& m, const MjbData& d, int w, int lane) {
+static __device__ void nxn_broadphase(const MjbModel& m, const MjbData& d, int w, int lane) {
   const float* gxpos = d.geom_xpos + W(w, 3 * m.ngeom);
   const float* gxmat = d.geom_xmat + W(w, 9 * m.ngeom);
   const int np = m.npair_cand;
@@ -186,7 +186,7 @@ __device__ __forceinline__ bool sap_overlap(float4 a, float4 b) {
   return rdot3(dx, dy, dz, dx, dy, dz) <= __fmul_rn(r, r);
 }
 
-__device__ void sap_broadphase(const MjbModel& m, const MjbData& d, int w, int lane, float* sm) {
+static __device__ void sap_broadphase(const MjbModel& m, const MjbData& d, int w, int lane, float* sm) {
   const int ng = m.ngeom, P = sap_pow2(ng);
   float4* S = reinterpret_cast<float4*>(sm);
   float* lo = sm + 4 * ng;
@@ -375,7 +375,7 @@ __device__ __forceinline__ void sphere_sphere_raw(ContactOut& o, f3 p1, float r1
 }
 
 // collision_primitive.py:235-268 for one candidate pair
-__device__ void narrow_pair(ContactOut& o) {
+static __device__ void narrow_pair(ContactOut& o) {
   const MjbModel& m = *o.m;
   const int g1 = o.g1, g2 = o.g2, w = o.w;
   const float* gxpos = o.d->geom_xpos + W(w, 3 * m.ngeom);
@@ -448,7 +448,7 @@ constexpr int kCountChunks = 21;
 
 // collision_primitive.py:271-274 over this world's pairs.  The world's contacts take one
 // contiguous block: a counting pass sizes it, a write pass fills it in pair order.
-__device__ void primitive_narrowphase(const MjbModel& m, const MjbData& d, int w, int lane) {
+static __device__ void primitive_narrowphase(const MjbModel& m, const MjbData& d, int w, int lane) {
   const int pa = d.world_pairadr[w], np = d.world_npair[w];
   int total = 0;
   unsigned long long counts = 0;
@@ -496,7 +496,7 @@ __device__ void primitive_narrowphase(const MjbModel& m, const MjbData& d, int w
 // collision_driver.py:525-547 (ngeom <= 100 path; larger models go through sap_broadphase, whose
 // pair set is the same set of overlapping candidates)
 // sm: sap_smem_floats(ngeom) floats of warp scratch when use_sap(m)
-__device__ void collision(const MjbModel& m, const MjbData& d, int w, int lane, float* sm) {
+static __device__ void collision(const MjbModel& m, const MjbData& d, int w, int lane, float* sm) {
   if (use_sap(m)) sap_broadphase(m, d, w, lane, sm);
   else nxn_broadphase(m, d, w, lane);
   primitive_narrowphase(m, d, w, lane);
@@ -518,7 +518,7 @@ __device__ __forceinline__ void root_dofs(const MjbModel& m, int root, int& a, i
 
 // ------------------------------------------------------------------------------------------
 // constraint.py:22-73
-__device__ void update_efc_row(const MjbModel& m, const MjbData& d, int r, float pos_aref,
+static __device__ void update_efc_row(const MjbModel& m, const MjbData& d, int r, float pos_aref,
                                float pos_imp, float invweight, const float* solref,
                                const float* solimp, float margin, bool refsafe, float Jqvel) {
   float timeconst = solref[0], dampratio = solref[1];
@@ -551,7 +551,7 @@ __device__ void update_efc_row(const MjbModel& m, const MjbData& d, int r, float
 }
 
 // constraint.py:213-240: joint limits (:104-141), then condim-3 pyramidal contacts (:144-210)
-__device__ void make_constraint(const MjbModel& m, const MjbData& d, int w, int lane) {
+static __device__ void make_constraint(const MjbModel& m, const MjbData& d, int w, int lane) {
   const int nv = m.nv;
   const bool on = !(m.disableflags & DSBL_CONSTRAINT);
   const bool do_lim = on && !(m.disableflags & DSBL_LIMIT) && m.nlimit > 0;

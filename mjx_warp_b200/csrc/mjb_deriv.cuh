@@ -33,7 +33,7 @@ __host__ __device__ __forceinline__ int fd_slots(const MjbModel& m, int flags) {
 
 // Writes base world w's state into perturbed slot pw and perturbs column col by delta (col < 0:
 // an unperturbed copy).
-__device__ void fd_perturb_world(const MjbModel& m, const MjbData& b, const MjbData& p, int w,
+static __device__ void fd_perturb_world(const MjbModel& m, const MjbData& b, const MjbData& p, int w,
                                  int pw, int col, float delta, int lane) {
   auto copy = [&](float* dst, const float* src, int n) {
     if (!dst || !src) return;
@@ -73,7 +73,7 @@ __device__ void fd_perturb_world(const MjbModel& m, const MjbData& b, const MjbD
 }
 
 // One column of A or B for base world w from the stepped perturbed batch.
-__device__ void fd_column(const MjbModel& m, const MjbData& p, int w, int col, int flags,
+static __device__ void fd_column(const MjbModel& m, const MjbData& p, int w, int col, int flags,
                           float eps, float* A, float* B, int lane) {
   const int centered = flags & kFdCentered;
   const int nv = m.nv, na = m.na, nx = 2 * nv + na, K = fd_slots(m, flags);
@@ -108,7 +108,7 @@ __device__ void fd_column(const MjbModel& m, const MjbData& p, int w, int col, i
 }
 
 // lam_out = A^T lam and grad_ctrl = B^T lam for world w (row-major A: nx x nx, B: nx x nu).
-__device__ void transition_vjp_world(const MjbModel& m, const float* A, const float* B,
+static __device__ void transition_vjp_world(const MjbModel& m, const float* A, const float* B,
                                      const float* lam, float* lam_out, float* grad_ctrl, int w,
                                      int lane) {
   const int nx = 2 * m.nv + m.na, nu = m.nu;
@@ -150,7 +150,7 @@ __host__ __device__ __forceinline__ int step_vjp_floats(const MjbModel& m, bool 
 // directly, and the adjoint of the velocity entering each dof's cdof_dot = v x cdof gets
 // qvel_i cdof_i x* G_b.  Walking every body's joints backwards (the order com_vel adds them in),
 // rq_i = G_b . cdof_dot_i + cdof_i . (adjoint of the body velocity after dof i's joint).
-__device__ void rne_vel_vjp(const MjbModel& m, const MjbData& d, int w, int lane, const float* s,
+static __device__ void rne_vel_vjp(const MjbModel& m, const MjbData& d, int w, int lane, const float* s,
                             const float* qvel, float* rq, float* U, float* G, float* R) {
   const int nb = m.nbody, nv = m.nv;
   const float* cdof = d.cdof + W(w, 6 * nv);
@@ -246,7 +246,7 @@ __device__ void rne_vel_vjp(const MjbModel& m, const MjbData& d, int w, int lane
 // lam_v (nv)) of the next state.  Any of grad_qpos / grad_qvel / grad_ctrl may be null.  One warp
 // per world (scratch: step_vjp_floats; for nv > 32 the Newton solver's factor of H in efc_h is
 // reused, and with CG H and its factor are written there), dense qM, na = 0.
-__device__ void step_vjp_world(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void step_vjp_world(const MjbModel& m, const MjbData& d, int w, int lane,
                                const float* lam, const float* qvel_prev, float* grad_ctrl,
                                float* grad_qvel, float* grad_qpos, float* tile) {
   const int nv = m.nv, nu = m.nu, nb = m.nbody, VL = step_vjp_vec(nv);

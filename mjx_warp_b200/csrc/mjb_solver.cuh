@@ -56,7 +56,7 @@ __device__ __forceinline__ void mul_m_ctx(SolverCtx& s, float* res, const float*
 }
 
 // solver.py:75-173
-__device__ void update_constraint(SolverCtx& s) {
+static __device__ void update_constraint(SolverCtx& s) {
   const MjbData& d = s.d;
   const int nv = s.nv;
   s.prev_cost = s.cost;
@@ -96,7 +96,7 @@ __device__ void update_constraint(SolverCtx& s) {
 // H = tril(qM) + sum over the world's active rows of D J'J: the lower triangle of the dense
 // nv x nv matrix at H (update_gradient's Newton Hessian, solver.py:249-276).  nz: null or
 // generic_nz_floats(nv) floats of warp scratch for the sparse-row assembly.
-__device__ void assemble_hessian(const MjbModel& m, const MjbData& d, const float* qM, float* H,
+static __device__ void assemble_hessian(const MjbModel& m, const MjbData& d, const float* qM, float* H,
                                  int adr, int n, float* nz, int lane) {
   const int nv = m.nv;
   if (nz) {
@@ -164,7 +164,7 @@ __device__ void assemble_hessian(const MjbModel& m, const MjbData& d, const floa
   }
 }
 
-__device__ void update_gradient(SolverCtx& s) {
+static __device__ void update_gradient(SolverCtx& s) {
   const MjbModel& m = s.m;
   const MjbData& d = s.d;
   const int nv = s.nv, lane = s.lane;
@@ -362,7 +362,7 @@ __device__ __forceinline__ void linesearch_with(SolverCtx& s, MulM&& mulm, RowDo
   __syncwarp();
 }
 
-__device__ void linesearch(SolverCtx& s) {
+static __device__ void linesearch(SolverCtx& s) {
   linesearch_with(s, [&]() { mul_m_ctx(s, s.mv, s.search); },
                   [&](int k) {
                     const float* J = s.d.efc_J + size_t(s.adr + k) * s.nv;
@@ -376,7 +376,7 @@ __device__ void linesearch(SolverCtx& s) {
 // solver.py:872-1000, any nv; hs: per-world nv*nv floats (the Newton Hessian and its factor);
 // nz: null or generic_nz_floats(nv) floats of warp scratch for the sparse-row Hessian assembly;
 // reuse: keep the factor while the active set is unchanged
-__device__ __noinline__ void solve_generic(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ __noinline__ void solve_generic(const MjbModel& m, const MjbData& d, int w, int lane,
                                            float* hs, float* nz, bool reuse) {
   const int nv = m.nv;
   SolverCtx s{m, d, w, lane, nv, d.world_efcadr[w], d.world_nefc[w]};

@@ -30,9 +30,10 @@ namespace mjb {
 // returns the totals.  red: K * NW elements of shared memory.
 template <int NW, int K, typename T>
 __device__ __forceinline__ void cta_sum(T (&v)[K], T* red, int warp, int lane) {
+  constexpr bool kEach = K < 4 || sizeof(T) == 8;  // (16 doubles would not stay in registers)
 #pragma unroll
-  for (int k = 0; K < 4 && k < K; k++) v[k] = warp_sum_t(v[k]);
-  if (K < 4) {
+  for (int k = 0; kEach && k < K; k++) v[k] = warp_sum_t(v[k]);
+  if constexpr (kEach) {
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < K; k++) red[k * NW + warp] = v[k];
@@ -1224,7 +1225,7 @@ __device__ __noinline__ void chol_cta_d(double* P, double* rd, int n, int warp, 
 // x = (L L^T)^-1 y for the packed FP64 factor in shared memory, one warp, in FP64 with the
 // intermediate vector in v (n doubles of shared memory) and the reciprocal diagonal rd; x and y
 // are n floats in global memory (x may alias y).
-__device__ void cho_solve_d_warp(const double* P, const double* rd, int n, double* v, float* x,
+static __device__ void cho_solve_d_warp(const double* P, const double* rd, int n, double* v, float* x,
                                  const float* y, int lane) {
   for (int i = lane; i < n; i += 32) v[i] = double(y[i]);
   __syncwarp();
@@ -1245,6 +1246,12 @@ __device__ void cho_solve_d_warp(const double* P, const double* rd, int n, doubl
   }
   for (int i = lane; i < n; i += 32) x[i] = float(v[i]);
   __syncwarp();
+}
+
+// the CG preconditioner, kept out of the Newton solver's code
+static __device__ __noinline__ void cta_solve_m(const MjbModel& m, const MjbData& d, int w, float* x,
+                                                const float* y, int lane) {
+  solve_m_world(m, d, w, x, y, lane);
 }
 
 template <int NW, bool PREC>
@@ -1271,6 +1278,8 @@ struct CtaSolver {
   float cost, prev_cost, gauss, grad_dot, search_dot, gtol, alpha, beta;
   float qg[3];
   static constexpr int NT = NW * 32;
+
+  __device__ __forceinline__ bool sparse() const { return !PREC && sp; }
 
   template <int K>
   __device__ __forceinline__ void sum(float (&v)[K]) { cta_sum<NW, K, float>(v, red, warp, lane); }
@@ -1316,7 +1325,7 @@ struct CtaSolver {
 #pragma unroll 1
     for (int i = tid; i < nv; i += NT) {
       int a, size;
-      if (sp) {
+      if (sparse()) {
         const int t = S->dtree[i];
         a = S->tadr[t];
         size = S->tadr[t + 1] - a;
@@ -1355,7 +1364,7 @@ struct CtaSolver {
 
   // out[r] = J_r . x - sub[r] for every row (warp per row); sub may be null
   __device__ void rows_dot(const float* x, float* out, const float* sub) {
-    if (sp && NW == 1) {
+    if (sparse() && NW == 1) {
 #pragma unroll 1
       for (int k = lane; k < n; k += 32) {
         const float v = row_dot(k, x);
@@ -1364,7 +1373,7 @@ struct CtaSolver {
       __syncwarp();
       return;
     }
-    if (sp) {
+    if (sparse()) {
       // Eight lanes per row over its trees' columns.  The dense form sums lane-strided partials
       // by a 32-lane butterfly; column c's partial belongs to lane c mod 32, so lane l of the eight
       // keeps the four partials l, l + 8, l + 16, l + 24 and adds them as the butterfly does.
@@ -1433,7 +1442,7 @@ struct CtaSolver {
       const int active = Jaref < 0.f;
       ch |= d.efc_active[r] != active;
       d.efc_active[r] = active;
-      if (sp) {
+      if (sparse()) {
         S->sD[k] = active ? D : 0.f;
         S->sF[k] = active ? -1.f * D * Jaref : 0.f;
       }
@@ -1448,7 +1457,7 @@ struct CtaSolver {
 #pragma unroll 1
     for (int i = tid; i < nv; i += NT) {
       float f = 0.f;
-      if (sp) {
+      if (sparse()) {
         const int t = S->dtree[i], a = S->tadr[t];
 #pragma unroll 1
         for (int e = S->radr[t]; e < S->radr[t + 1]; e++) {
@@ -1458,7 +1467,7 @@ struct CtaSolver {
         }
       }
 #pragma unroll 1
-      for (int k = sp ? n : 0; k < n; k++) {
+      for (int k = sparse() ? n : 0; k < n; k++) {
         const float fk = d.efc_force[adr + k];
         if (fk != 0.f) f += d.efc_J[size_t(adr + k) * nv + i] * fk;
       }
@@ -1722,7 +1731,7 @@ struct CtaSolver {
     sum<1>(gd);
     grad_dot = gd[0];
     if (m.solver == 1) {  // CG: Mgrad = M^-1 grad
-      if (warp == 0) solve_m_world(m, d, w, Mgrad, grad, lane);
+      if (warp == 0) cta_solve_m(m, d, w, Mgrad, grad, lane);
       __syncthreads();
       return;
     }
@@ -1736,7 +1745,7 @@ struct CtaSolver {
           if (j <= i) H[e] = float(Ld[tri(i) + j]);
         }
       } else {
-        if (sp) {
+        if (sparse()) {
           assemble_hessian_sparse();
           chol_cta_sparse<NW, SH>(nv, T, *S, warp, lane);
         } else if constexpr (NW > 1) {
@@ -1750,7 +1759,7 @@ struct CtaSolver {
     if (warp == 0) {
       if (PREC) cho_solve_d_warp(Ld, rdg, nv, vd, Mgrad, grad, lane);
     }
-    if (!PREC && sp) cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
+    if (sparse()) cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
     else if constexpr (!PREC && NW > 1) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
     __syncthreads();
   }
@@ -2034,7 +2043,7 @@ struct CtaSolver {
       const float scale = m.meaninertia * float(max(1, nv));
       done = it >= 0 && ((prev_cost - cost) / scale < m.tolerance || sqrtf(grad_dot) / scale < m.tolerance);
     }
-    if (sp && factored && S->L != H) store_factor();
+    if (sparse() && factored && S->L != H) store_factor();
     float* wsw = d.qacc_warmstart + W(w, nv);
 #pragma unroll 1
     for (int i = tid; i < nv; i += NT) wsw[i] = qacc[i];

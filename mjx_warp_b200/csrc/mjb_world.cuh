@@ -245,7 +245,7 @@ __device__ __forceinline__ int madr_row_len(const MjbModel& m, int i) {
 
 // smooth.py:317-351 (mj_factorI): in-place L'DL, each tree's dofs eliminated from its last to its
 // first, each elimination updating its ancestors' rows; Dinv (may be null) = 1 / D
-__device__ void factor_sparse(const MjbModel& m, float* L, float* Dinv, int lane) {
+static __device__ void factor_sparse(const MjbModel& m, float* L, float* Dinv, int lane) {
   for (int blk = lane; blk < m.nblock; blk += 32) {
     const int a = m.block_adr[blk], n = m.block_size[blk];
     for (int k = a + n - 1; k >= a; k--) {
@@ -267,7 +267,7 @@ __device__ void factor_sparse(const MjbModel& m, float* L, float* Dinv, int lane
 // x = M^-1 y from the L'DL factor (smooth.py:609-652, mj_solveLD): x <- L'^-1 x from the leaves
 // up, x <- D^-1 x, x <- L^-1 x from the roots down.  Dinv may be null (1 / D is then formed from
 // L).  x may alias y.
-__device__ void solve_sparse(const MjbModel& m, const float* L, const float* Dinv, float* x,
+static __device__ void solve_sparse(const MjbModel& m, const float* L, const float* Dinv, float* x,
                              const float* y, int lane) {
   for (int blk = lane; blk < m.nblock; blk += 32) {
     const int a = m.block_adr[blk], n = m.block_size[blk];
@@ -287,7 +287,7 @@ __device__ void solve_sparse(const MjbModel& m, const float* L, const float* Din
 
 // res = M vec for the sparse M (support.py:96-137: the diagonal, then each stored off-diagonal
 // entry applied to both of its rows); res must not alias vec
-__device__ void mul_m_sparse(const MjbModel& m, const float* M, float* res, const float* vec,
+static __device__ void mul_m_sparse(const MjbModel& m, const float* M, float* res, const float* vec,
                              int lane) {
   for (int blk = lane; blk < m.nblock; blk += 32) {
     const int a = m.block_adr[blk], n = m.block_size[blk];
@@ -304,7 +304,7 @@ __device__ void mul_m_sparse(const MjbModel& m, const float* M, float* res, cons
 }
 
 // Scatters the sparse M into the lower triangle of a dense nv x nv matrix H (upper left alone)
-__device__ void sparse_to_lower(const MjbModel& m, const float* M, float* H, int lane) {
+static __device__ void sparse_to_lower(const MjbModel& m, const float* M, float* H, int lane) {
   const int nv = m.nv;
   for (int e = lane; e < nv * nv; e += 32) {
     const int i = e / nv, j = e - i * nv;
@@ -437,7 +437,7 @@ __device__ __noinline__ void chol_lower(T* A, int ld, int n, int lane) {
 // per-warp buffer and subtracts L[i][k] * L[j][k] from the rest of its row — independent FMAs fed
 // by broadcast reads.  On exit L holds the factor; the return value is (1 / L[i][i], z_i) with
 // z = L^-1 y for the lane's y_i (0 for lanes >= n).  Blocks of up to 4 warps (one buffer each).
-__device__ __noinline__ float2 chol32(float* L, int ldl, int n, int lane, float y) {
+static __device__ __noinline__ float2 chol32(float* L, int ldl, int n, int lane, float y) {
   __shared__ float colbuf[4][32];
   float* col = colbuf[(threadIdx.x >> 5) & 3];
   float r[32];
@@ -544,7 +544,7 @@ __device__ __forceinline__ void copy_rows(const float* src, int sld, float* dst,
 // and one __syncwarp() publishes the four columns.  Every sum is formed in the order of the
 // one-column form (the same float4 chunks, then the remaining terms in column order into the first
 // partial sum), so the factor is the same bit for bit.
-__device__ MJB_TILE_FN void chol_tile(float* A, int ld, int n, int lane) {
+static __device__ MJB_TILE_FN void chol_tile(float* A, int ld, int n, int lane) {
   float* Ar = A + min(lane, n - 1) * ld;  // lanes past the last row repeat it
   for (int k = 0; k < n; k += 4) {
     const int nb = min(4, n - k);  // columns of this step
@@ -584,7 +584,7 @@ __device__ MJB_TILE_FN void chol_tile(float* A, int ld, int n, int lane) {
 // group, 0 for lanes past the last row): every group takes its own four-column steps, so the tile
 // takes as many steps as its largest group instead of n / 4.  The columns outside a row's group are
 // zero, so each sum is chol_tile's.
-__device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned g, int lane) {
+static __device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned g, int lane) {
   float* Ar = A + min(lane, n - 1) * ld;
   unsigned cm = 0u;  // four-column chunks with columns of the group
 #pragma unroll
@@ -634,7 +634,7 @@ __device__ __noinline__ void chol_tile_groups(float* A, int ld, int n, unsigned 
 // x = (L L^T)^-1 y for an n <= 32 tile factor; lane i holds y_i and returns x_i (the arithmetic of
 // cho_solve32).  The forward pass reads the lane's own row four columns at a time, the backward
 // pass row k across the lanes; neither load depends on the substitution chain.
-__device__ MJB_TILE_FN float cho_solve_tile(const float* L, int ld, int n, float y, int lane) {
+static __device__ MJB_TILE_FN float cho_solve_tile(const float* L, int ld, int n, float y, int lane) {
   const bool own = lane < n;
   const float* Li = L + min(lane, n - 1) * ld;
   const float invd = own ? __frcp_rn(Li[lane]) : 0.f;
@@ -670,7 +670,7 @@ __device__ MJB_TILE_FN float cho_solve_tile(const float* L, int ld, int n, float
 // columns (pairs of partial sums, k a multiple of 4) feeds the four columns, then column k + j
 // adds the terms of columns k .. k + j - 1 as the one-column form orders them (the pair
 // (k, k + 1) into the two partial sums, column k + 2 as the tail term).
-__device__ __noinline__ void chol_tile_d(double* A, int ld, int n, int lane) {
+static __device__ __noinline__ void chol_tile_d(double* A, int ld, int n, int lane) {
   double* Ar = A + min(lane, n - 1) * ld;  // lane i on row i; lanes past the last row repeat it
   for (int k = 0; k < n; k += 4) {
     const int nb = min(4, n - k);
@@ -705,7 +705,7 @@ __device__ __noinline__ void chol_tile_d(double* A, int ld, int n, int lane) {
 }
 // The substitutions multiply by each lane's reciprocal pivot, formed once (one FP64 division per
 // lane instead of one per step of each pass); lane k scales its entry, one shuffle broadcasts it.
-__device__ __noinline__ double cho_solve_tile_d(const double* L, int ld, int n, double y, int lane) {
+static __device__ __noinline__ double cho_solve_tile_d(const double* L, int ld, int n, double y, int lane) {
   const bool own = lane < n;
   const double* Li = L + min(lane, n - 1) * ld;
   const double invd = own ? 1.0 / Li[lane] : 0.0;
@@ -725,7 +725,7 @@ __device__ __noinline__ double cho_solve_tile_d(const double* L, int ld, int n, 
   return own ? x : 0.0;
 }
 // chol_tile_d group by group, as chol_tile_groups
-__device__ __noinline__ void chol_tile_d_groups(double* A, int ld, int n, unsigned g, int lane) {
+static __device__ __noinline__ void chol_tile_d_groups(double* A, int ld, int n, unsigned g, int lane) {
   double* Ar = A + min(lane, n - 1) * ld;
   unsigned cm = 0u;
 #pragma unroll
@@ -853,7 +853,7 @@ __device__ __forceinline__ void tile_store_lower(const float* T, int tld, int n,
 // broadcast); (c) the trailing lower triangle is updated, A_ij -= L_i . L_j over the panel, one
 // chunk of 32 rows j at a time staged in T, lane per row i, float4 broadcast reads.  The column
 // dot products are accumulated panel by panel, so the bits differ from chol_lower's.
-__device__ __noinline__ void chol_blocked(float* A, int ld, int n, int lane, float* T) {
+static __device__ __noinline__ void chol_blocked(float* A, int ld, int n, int lane, float* T) {
   constexpr int TL = 36;
   for (int p0 = 0; p0 < n; p0 += 32) {
     const int pn = min(32, n - p0);
@@ -926,7 +926,7 @@ __device__ __forceinline__ void chol_any(float* A, int ld, int n, int lane, floa
 }
 
 // x = (L L^T)^-1 y for the n x n lower factor at L (leading dimension ld); x may alias y.
-__device__ void warp_cho_solve(const float* L, int ld, int n, float* x, const float* y, int lane) {
+static __device__ void warp_cho_solve(const float* L, int ld, int n, float* x, const float* y, int lane) {
   if (n <= 32) {
     float xi = lane < n ? y[lane] : 0.f;
     for (int k = 0; k < n; k++) {  // L z = y
@@ -969,7 +969,7 @@ __device__ void warp_cho_solve(const float* L, int ld, int n, float* x, const fl
 // into L (smooth.py:353-379, qLD_tile semantics; zeros outside the blocks' lower triangles).  With
 // a per-warp tile, blocks of n <= 32 are factored in shared memory and written back row by row;
 // the tile then holds the factor of the last block.
-__device__ void factor_blocks(const MjbModel& m, const float* M, float* L, int lane,
+static __device__ void factor_blocks(const MjbModel& m, const float* M, float* L, int lane,
                               const float* dadd = nullptr, float scale = 0.f, float* tile = nullptr) {
   const int nv = m.nv;
   // one tiled block covering every dof is written whole by tile_store_lower
@@ -1034,7 +1034,7 @@ __device__ void factor_blocks(const MjbModel& m, const float* M, float* L, int l
 // x = M^-1 y per tree block from the block factor L (smooth.py:654-681); x may alias y.  With a
 // tile, blocks of n <= 32 are staged into it row by row first, unless tile_has_factor says that
 // the tile already holds the factor of the model's only block.
-__device__ void solve_blocks(const MjbModel& m, const float* L, float* x, const float* y,
+static __device__ void solve_blocks(const MjbModel& m, const float* L, float* x, const float* y,
                              int lane, float* tile = nullptr, bool tile_has_factor = false) {
   const int nv = m.nv;
   for (int blk = 0; blk < m.nblock; blk++) {
@@ -1084,7 +1084,7 @@ __device__ void solve_blocks(const MjbModel& m, const float* L, float* x, const 
 
 // x = (M + scale diag(dadd))^-1 y per tree block, factored and solved in FP64 in the double tile
 // dt (precision form; blocks of n <= 32, dense M with leading dimension nv).
-__device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, const float* dadd,
+static __device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, const float* dadd,
                                       float scale, float* x, const float* y, int lane, double* dt) {
   const int nv = m.nv, ld = tile_ld(nv);
   for (int blk = 0; blk < m.nblock; blk++) {
@@ -1129,7 +1129,7 @@ __device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, const f
 }
 
 // smooth.py:392-395
-__device__ void factor_m(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
+static __device__ void factor_m(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv;
   if (m.is_sparse) {  // smooth.py:317-351
     const float* M = d.qM + W(w, m.nM);
@@ -1399,7 +1399,7 @@ __device__ void fwd_actuation(const MjbModel& m, const MjbData& d, int w, int la
 }
 
 // support.py:140-172 — qfrc += J^T xfrc_applied (Jacobian at each body's xipos)
-__device__ void xfrc_accumulate(const MjbModel& m, const MjbData& d, int w, float* qfrc, int lane) {
+static __device__ void xfrc_accumulate(const MjbModel& m, const MjbData& d, int w, float* qfrc, int lane) {
   const int nv = m.nv, nb = m.nbody;
   const float* cdof = d.cdof + W(w, 6 * nv);
   const float* xipos = d.xipos + W(w, 3 * nb);
@@ -1426,7 +1426,7 @@ __device__ void xfrc_accumulate(const MjbModel& m, const MjbData& d, int w, floa
 
 // forward.py:644-661
 // tile_has_qLD: the per-warp tile still holds the factor left by factor_m
-__device__ void fwd_acceleration(const MjbModel& m, const MjbData& d, int w, int lane,
+static __device__ void fwd_acceleration(const MjbModel& m, const MjbData& d, int w, int lane,
                                  float* tile = nullptr, bool tile_has_qLD = false) {
   const int nv = m.nv;
   float* sm = d.qfrc_smooth + W(w, nv);
@@ -1447,7 +1447,7 @@ __device__ void fwd_acceleration(const MjbModel& m, const MjbData& d, int w, int
 
 // ------------------------------------------------------------------------------------------
 // forward.py:43-162 — advance velocities and positions (semi-implicit)
-__device__ void advance(const MjbModel& m, const MjbData& d, int w, const float* qacc, int lane) {
+static __device__ void advance(const MjbModel& m, const MjbData& d, int w, const float* qacc, int lane) {
   const int nv = m.nv;
   const float dt = m.timestep;
   float* qvel = d.qvel + W(w, nv);
@@ -1469,7 +1469,7 @@ __device__ void advance(const MjbModel& m, const MjbData& d, int w, const float*
 }
 
 // forward.py:165-242 — Euler with implicit joint damping unless EULERDAMP is disabled
-__device__ void euler(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
+static __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv;
   if (m.disableflags & DSBL_EULERDAMP) {
     advance(m, d, w, d.qacc + W(w, nv), lane);
@@ -1515,7 +1515,7 @@ __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lane, floa
 
 // forward.py:245-405 — implicitfast (dense): (M - dt qDeriv) qacc = qfrc_smooth + qfrc_constraint
 // with qDeriv = moment^T diag(bias_vel + gain_vel * ctrl) moment - diag(damping)
-__device__ void implicit(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
+static __device__ void implicit(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv, nu = m.nu;
   const bool passive_on = !(m.disableflags & DSBL_PASSIVE);
   const bool act_on = !(m.disableflags & DSBL_ACTUATION) && m.actuator_affine_bias_gain;
