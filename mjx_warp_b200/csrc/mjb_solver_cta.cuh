@@ -1248,6 +1248,49 @@ static __device__ void cho_solve_d_warp(const double* P, const double* rd, int n
   __syncwarp();
 }
 
+// cho_solve_d_warp for n <= 128: the vector in four registers per lane (entry i on lane i mod 32), each
+// entry broadcast by a shuffle, instead of a column step through shared memory between two warp
+// barriers: the same operations on every entry in the same order.
+static __device__ __noinline__ void cho_solve_d_regs(const double* P, const double* rd, int n, float* x,
+                                                     const float* y, int lane) {
+  double v[4];
+  const double* R[4];  // the lane's rows
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    const int i = lane + 32 * t;
+    v[t] = i < n ? double(y[i]) : 0.0;
+    R[t] = P + tri(min(i, n - 1));
+  }
+#pragma unroll
+  for (int b = 0; b < 4; b++) {  // L z = y
+#pragma unroll 1
+    for (int k = 32 * b; k < min(n, 32 * b + 32); k++) {
+      const double zk = __shfl_sync(WARP_FULL, v[b], k & 31) * rd[k];
+      if (lane + 32 * b == k) v[b] = zk;
+      else if (lane + 32 * b > k && lane + 32 * b < n) v[b] -= R[b][k] * zk;
+#pragma unroll
+      for (int t = b + 1; t < 4; t++)
+        if (lane + 32 * t < n) v[t] -= R[t][k] * zk;
+    }
+  }
+#pragma unroll
+  for (int b = 3; b >= 0; b--) {  // L^T x = z
+#pragma unroll 1
+    for (int k = min(n, 32 * b + 32) - 1; k >= 32 * b; k--) {
+      const double xk = __shfl_sync(WARP_FULL, v[b], k & 31) * rd[k];
+      const double* Lk = P + tri(k) + lane;
+      if (lane + 32 * b == k) v[b] = xk;
+      else if (lane + 32 * b < k) v[b] -= Lk[32 * b] * xk;
+#pragma unroll
+      for (int t = 0; t < b; t++) v[t] -= Lk[32 * t] * xk;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 4; t++)
+    if (lane + 32 * t < n) x[lane + 32 * t] = float(v[t]);
+  __syncwarp();
+}
+
 // the CG preconditioner, kept out of the Newton solver's code
 static __device__ __noinline__ void cta_solve_m(const MjbModel& m, const MjbData& d, int w, float* x,
                                                 const float* y, int lane) {
@@ -1757,7 +1800,8 @@ struct CtaSolver {
       factored = true;
     }
     if (warp == 0) {
-      if (PREC) cho_solve_d_warp(Ld, rdg, nv, vd, Mgrad, grad, lane);
+      if (PREC && nv <= 128) cho_solve_d_regs(Ld, rdg, nv, Mgrad, grad, lane);
+      else if (PREC) cho_solve_d_warp(Ld, rdg, nv, vd, Mgrad, grad, lane);
     }
     if (sparse()) cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
     else if constexpr (!PREC && NW > 1) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
