@@ -151,7 +151,7 @@ def _algorithmic_bytes(d, mjm, ncon, nefc):
 
 
 FORMS = {"plain": 0, "chosen": 1, "single": 2, "precision": 3}
-LAUNCHES = {"plain": 16, "chosen": 16, "single": 2, "precision": 16}  # kernels per step (mjb200.cu run_* paths)
+LAUNCHES = {"plain": 16, "chosen": 15, "single": 2, "precision": 15}  # kernels per step (mjb200.cu run_* paths)
 
 
 def _solver_bytes(mjm, nworld, nefc):
