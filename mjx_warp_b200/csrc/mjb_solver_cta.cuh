@@ -362,7 +362,7 @@ struct SparseShape {
   uint8_t ntree[kNodes];                 // its tree
   uint8_t dtree[kDofs];                  // tree of each dof
   SparseOrder<kNodes> fwd, bwd;
-  int nblk, bad, compact;
+  int nblk, compact;
   unsigned cnt[kSpTrees];
 
   // column of tree u's first dof in tree t's rows of L
@@ -392,7 +392,8 @@ __device__ __forceinline__ unsigned panel_bits(const SH& S, int u, int c0, int p
 }
 
 // Finds the structure of a world's n rows (J: n x nv dense) by a CTA of NW warps; false (in every
-// thread) when it does not fit the masks or lists, and the dense routines then run.  cw: floats per
+// thread) when it does not fit the masks or lists, and the dense routines then run.  Whether it fits
+// is decided by the reduction of a barrier: every warp returns from the same one.  cw: floats per
 // row of cj (twice the largest tree), or 0 when the rows do not fit there.  H: the world's efc_h.
 template <int NW, class SH>
 __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int n, float* H,
@@ -402,7 +403,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
   if (n > SH::kRows) return false;
   cw = 2 * m.block_max;
   if (n * cw > SH::kJ) cw = 0;
-  if (tid == 0) S.bad = 0;
+  bool bad = false;  // what this thread found does not fit
 #pragma unroll 1
   for (int t = tid; t < nt; t += NT) {
     const int a = m.block_adr[t], z = m.block_size[t];
@@ -465,7 +466,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
       const int c = __popcll(mk);
       const int u = mk ? __ffsll(mk) - 1 : 0, t = mk ? 63 - __clzll(mk) : 0;
       if (lane == 0) {
-        if (c > 2) S.bad = 1;
+        if (c > 2) bad = true;
         S.rtree[k] = uint16_t(u | (t << 8));
         atomicAdd(&S.cnt[t], 1u);
         if (u != t) {
@@ -482,8 +483,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
       }
     }
   }
-  __syncthreads();
-  if (S.bad) return false;
+  if (__syncthreads_or(bad)) return false;
   if (warp == 0) {  // elimination fill, tree by tree; lane l holds trees l and l + 32
     unsigned long long m0 = lane < nt ? S.tmask[lane] : 0ull;
     unsigned long long m1 = lane + 32 < nt ? S.tmask[lane + 32] : 0ull;
@@ -503,10 +503,8 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
     const int e0 = warp_excl_scan(__popcll(m0), lane, &tot0);
     const int e1 = warp_excl_scan(__popcll(m1), lane, &tot1) + tot0;
     const bool fits = tot0 + tot1 <= SH::kBlocks;
-    if (lane == 0) {
-      S.nblk = tot0 + tot1;
-      if (!fits) S.bad = 1;
-    }
+    bad = !fits;
+    if (lane == 0) S.nblk = tot0 + tot1;
     int w0 = 0, w1 = 0;  // columns of this lane's trees
     if (fits) {
       S.bst[lane] = uint16_t(e0);
@@ -552,8 +550,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
     S.radr[lane + 32] = uint16_t(a1);
     if (lane == 0) S.radr[kSpTrees] = uint16_t(tot0 + tot1);
   }
-  __syncthreads();
-  if (S.bad) return false;
+  if (__syncthreads_or(bad)) return false;
 #pragma unroll 1
   for (int t = warp; t < nt; t += NW) {  // rows of each tree, ascending
     int e = S.radr[t];
@@ -638,10 +635,8 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
         at += tot;
       }
     }
-    if (lane == 0) {
-      S.padr[n32] = uint16_t(min(at, SH::kSlots));
-      if (at > SH::kSlots) S.bad = 1;
-    }
+    if (lane == 0) S.padr[n32] = uint16_t(min(at, SH::kSlots));
+    bad = at > SH::kSlots;
   }
   if (warp == NW - 1) {  // the tiles that earlier panels update: the pairs with a common earlier tree
     int at = 0;
@@ -673,13 +668,10 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
           }
       }
     }
-    if (lane == 0) {
-      S.iadr[n32] = uint16_t(min(at, SH::kItems));
-      if (at > SH::kItems) S.bad = 1;
-    }
+    if (lane == 0) S.iadr[n32] = uint16_t(min(at, SH::kItems));
+    bad |= at > SH::kItems;
   }
-  __syncthreads();
-  if (S.bad) return false;
+  if (__syncthreads_or(bad)) return false;
   // Levels: a node waits for every node of the trees its rows (forward) or columns (backward) couple
   // with, and for its own tree's previous node.  Warp 0 takes the forward order, warp 1 the other.
 #pragma unroll 1

@@ -1,6 +1,6 @@
 """The solver of models of several kinematic trees (nv > 32) over nonzero trees and tiles only, at the
 edges of its structure: 2 to 65 trees (64 is the most that it takes), tree sizes 6 and 27, matrices
-whose last 32-dof panel is partial, worlds without rows, rows past its row capacity."""
+whose last 32-dof panel is partial, worlds without rows, rows and tree pairs past its capacities."""
 
 import numpy as np
 import pytest
@@ -39,16 +39,33 @@ def case(name):
     q, v, u, _ = humanoid_spheres_state(mjm, load("humanoid.xml"), 8, seed=3)
     return mjm, q, v, u, 384
   mjm = load("bin.xml", **opt)
-  q, v, u = bin_state(mjm, 4, seed=6)
+  q, v, u = bin_state(mjm, 4, seed=3 if name == "bin_pairs" else 6)
+  x = q.reshape(4, -1, 7)
   if name == "bin_rows":  # every body in one heap in worlds 0 and 1
-    x = q.reshape(4, -1, 7)
     x[:2, :, :3] = np.array([0.0, 0.0, 0.3]) + 0.28 * (x[:2, :, :3] - np.array([0.0, 0.0, 0.19]))
+  if name == "bin_pairs":  # heaps of 477 to 624 tree pairs
+    x[:, :, :3] = np.array([0.0, 0.0, 0.3]) + 0.5 * (x[:, :, :3] - np.array([0.0, 0.0, 0.19]))
   return mjm, q, v, u, 2048
+
+
+def tree_pairs(mjm, J):
+  """Nonzero tree pairs of the factor of H for the rows J: each tree with itself, with the trees that
+  a row couples it with, and the fill of eliminating the trees in dof order."""
+  tree = np.asarray(mjm.dof_bodyid)
+  tree = np.unique(np.asarray(mjm.body_rootid)[tree], return_inverse=True)[1]
+  n = tree.max() + 1
+  touch = np.zeros((len(J), n), dtype=np.int64)
+  np.maximum.at(touch.T, tree, (J != 0).T.astype(np.int64))
+  C = (touch.T @ touch > 0) | np.eye(n, dtype=bool)
+  for k in range(n):
+    later = np.nonzero(C[k + 1:, k])[0] + k + 1
+    C[np.ix_(later, later)] = True
+  return int(np.tril(C).sum())
 
 
 @pytest.mark.parametrize("warps", [2, 4])
 @pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres64", "spheres65", "humanoid_spheres",
-                                  "bin", "bin_rows"])
+                                  "bin", "bin_rows", "bin_pairs"])
 def test_factor_of_the_hessian(name, warps):
   """With no iterations efc_h is the factor of H = qM + J_a' D_a J_a at the warmstart's active set:
   zero where H's factor is, and L L' = H within the backward error of an FP32 Cholesky factorisation
@@ -69,6 +86,10 @@ def test_factor_of_the_hessian(name, warps):
     assert n.max() > 736 > n.min()
   J, D = (x.cpu().numpy().astype(np.float64) for x in (d.efc.J, d.efc.D))
   act = d.efc.active.cpu().numpy().astype(bool)
+  if name == "bin_pairs":  # more pairs than the structure's 512 with no more than its 736 rows, and fewer
+    first = np.cumsum(n) - n
+    pairs = np.array([tree_pairs(mjm, J[idx[a:a + k]]) for a, k in zip(first, n)])
+    assert np.any((pairs > 512) & (n <= 736)) and np.any((pairs <= 512) & (n <= 736)), (pairs, n)
   at = 0
   for w in range(nworld):
     rows = idx[at:at + n[w]]
