@@ -633,13 +633,7 @@ static __device__ void make_constraint(const MjbModel& m, const MjbData& d, int 
     const float* sc = d.subtree_com + W(w, 3 * m.nbody);
     const bool trees = nv > 32;  // rows zeroed first, then written over the bodies' trees
     if (trees) {
-      float* J = d.efc_J + size_t(adr + nlim) * nv;
-      const size_t cnt = size_t(4 * ncact) * nv;
-      if ((nv & 3) == 0) {
-        for (size_t e = lane; e < cnt / 4; e += 32) reinterpret_cast<float4*>(J)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        for (size_t e = lane; e < cnt; e += 32) J[e] = 0.f;
-      }
+      zero_fill<32>(d.efc_J + size_t(adr + nlim) * nv, size_t(4 * ncact) * nv, lane);
       __syncwarp();
     }
     // nv <= 32: the lane's dof is the same for every contact

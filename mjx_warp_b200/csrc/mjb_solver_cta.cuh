@@ -185,7 +185,7 @@ __device__ __noinline__ void chol_cta(float* A, int ld, int n, float* T, int war
       if (lane < pn) T[lane * TL + 32] = __frcp_rn(T[lane * TL + lane]);
     }
     __syncthreads();
-    const bool vec = (ld & 3) == 0 && pn == 32;  // rows 16-byte aligned: float4 reads and writes
+    const bool vec = (ld & 3) == 0 && pn == 32 && aligned16(A);  // rows 16-byte aligned: float4 reads and writes
     for (int i = c0 + pn + int(threadIdx.x); i < n; i += NW * 32) {  // (iii)
       float* Ai = A + size_t(i) * ld + c0;
       float x[32];
@@ -417,7 +417,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
   __syncthreads();
   // rows: a warp per four rows, four columns per lane of each loaded at once; the trees of the
   // nonzero entries
-  const bool v4 = (nv & 3) == 0;
+  const bool v4 = (nv & 3) == 0 && aligned16(J);
 #pragma unroll 1
   for (int k0 = 4 * warp; k0 < n; k0 += 4 * NW) {
     unsigned lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u};
@@ -1554,7 +1554,7 @@ struct CtaSolver {
       for (int i = warp; i < nv; i += NW) {
         float* Hi = H + size_t(i) * nv;
         int j0 = 0;
-        if ((nv & 3) == 0) {
+        if ((nv & 3) == 0 && aligned16(H)) {
           j0 = (i + 1) & ~3;
 #pragma unroll 1
           for (int j = 4 * lane; j < j0; j += 128) *reinterpret_cast<float4*>(Hi + j) = make_float4(0.f, 0.f, 0.f, 0.f);

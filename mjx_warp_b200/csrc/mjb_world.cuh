@@ -43,13 +43,16 @@ __device__ __forceinline__ void lsync() {
   else __syncwarp(((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)));
 }
 
+// The caller's arrays start at any multiple of 4 bytes: a 16-byte access looks at the address first.
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<size_t>(p) & 15) == 0; }
+
 // zeros into p[0 .. n) by L lanes, 16 bytes a lane where p allows it
-template <int L>
-__device__ __forceinline__ void zero_fill(float* p, int n, int lane) {
-  int e = 0;
-  if ((reinterpret_cast<size_t>(p) & 15) == 0) {
-    e = n & ~3;
-    for (int i = lane; i < n / 4; i += L) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+template <int L, class N>
+__device__ __forceinline__ void zero_fill(float* p, N n, int lane) {
+  N e = 0;
+  if (aligned16(p)) {
+    e = n / 4 * 4;
+    for (N i = lane; i < n / 4; i += L) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   for (e += lane; e < n; e += L) p[e] = 0.f;
 }

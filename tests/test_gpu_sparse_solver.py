@@ -127,3 +127,27 @@ def test_one_warp_form_equals_plain(name):
   for f in ("cost", "Ma", "h"):
     a, b = getattr(out[1].efc, f), getattr(out[0].efc, f)
     assert torch.equal(a.tril(), b.tril()) if f == "h" else torch.equal(a, b), f
+
+
+@pytest.mark.parametrize("name", ["spheres6", "spheres66", "bin"])
+def test_rows_and_hessian_at_any_address(name):
+  """efc.J and efc.h as contiguous views at a 4-byte offset give what 16-byte aligned ones give: the
+  one-warp form (6 spheres), the dense one (66 trees, nv a multiple of 4) and the sparse one."""
+  mjm, q, v, u, cap = case(name)
+  mjm.opt.iterations = 10
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  out = []
+  for offset in (0, 1):
+    d = device_data(mjm, q, v, u, nconmax=800 * nworld, njmax=cap * nworld)
+    for f in ("J", "h"):
+      t = getattr(d.efc, f)
+      base = torch.zeros(t.numel() + 4, device="cuda")
+      setattr(d.efc, f, base[offset:offset + t.numel()].view(t.shape))
+      assert getattr(d.efc, f).data_ptr() % 16 == 4 * offset
+    mjw.forward(m, d)
+    torch.cuda.synchronize()
+    assert np.all(mjw.world_status(d) == 0)
+    out.append((d.efc.J.cpu()[world_rows(d, "efc")[1]], d.efc.h.cpu().tril(), d.qacc.cpu()))
+  for a, b in zip(*out):
+    assert torch.equal(a, b)
