@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(NW * 32, NW >= 16 ? 1 : (NW >= 8 ? 2 : (NW >= 
 
 template <int NW, bool PREC>
 inline void launch_cta(const MjbModel* m, const MjbData* d, int tc, cudaStream_t s) {
-  const size_t bytes = size_t(cta_solver_smem_floats(m->nv, NW, PREC)) * sizeof(float);
+  const size_t bytes = size_t(cta_solver_smem_floats(m->nv, NW, PREC, sparse_launch<NW, PREC>(*m, tc != 0))) * sizeof(float);
   static size_t conf[kSmemDevices];
   allow_smem(k_solve_cta<NW, PREC>, bytes, conf);
   if (d->world_order && d->work_queue && d->world_nefc) {

@@ -10,6 +10,6 @@ void launch_solver_cta_prec(const MjbModel* m, const MjbData* d, int nw, cudaStr
   else launch_cta<8, true>(m, d, 0, s);
 }
 
-size_t solver_cta_prec_smem(int nv) { return size_t(cta_solver_smem_floats(nv, 16, true)) * sizeof(float); }
+size_t solver_cta_prec_smem(int nv) { return size_t(cta_solver_smem_floats(nv, 16, true, false)) * sizeof(float); }
 
 }  // namespace mjb

@@ -2,6 +2,8 @@
 edges of its structure: 2 to 65 trees (64 is the most that it takes), tree sizes 6 and 27, matrices
 whose last 32-dof panel is partial, worlds without rows, rows and tree pairs past its capacities."""
 
+import json
+
 import numpy as np
 import pytest
 import torch
@@ -21,6 +23,15 @@ def spheres_xml(n):
     f'<geom type="sphere" size="0.1"/></body>' for i in range(n))
   return ('<mujoco><option timestep="0.002"/><worldbody><geom type="plane" size="0 0 1"/>'
           + bodies + "</worldbody></mujoco>")
+
+
+def chain_xml(n):
+  """One tree: a chain of n hinges whose links touch the plane below them only."""
+  s = '<mujoco><option timestep="0.002"/><worldbody><geom type="plane" size="0 0 1" pos="0 0 -0.1"/>'
+  for i in range(n):
+    s += (f'<body pos="{0.1 if i else 0} 0 0"><joint type="hinge" damping="0.3" axis="{i % 2} {(i + 1) % 2} 0.2"/>'
+          '<geom type="capsule" fromto="0 0 0 0.1 0 0" size="0.02" contype="0" conaffinity="1"/>')
+  return s + "</body>" * n + "</worldbody></mujoco>"
 
 
 def case(name):
@@ -151,3 +162,32 @@ def test_rows_and_hessian_at_any_address(name):
     out.append((d.efc.J.cpu()[world_rows(d, "efc")[1]], d.efc.h.cpu().tril(), d.qacc.cpu()))
   for a, b in zip(*out):
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name, tc", [("chain40", False), ("spheres66", False), ("spheres11", True)])
+def test_dense_launches_keep_their_shared_memory(name, tc, tmp_path):
+  """One tree, more than 64 trees and the tensor-core assembly do not look for a structure: their launch
+  asks for the dense form's shared memory only, and eight two-warp blocks fit on an SM (228 KB, 1 KB of
+  each block's reserved)."""
+  if name.startswith("chain"):
+    mjm = load(chain_xml(int(name[5:])), jacobian=MJ_JAC_DENSE)
+    q, v, u = np.tile(mjm.qpos0, (5, 1)), np.zeros((5, mjm.nv)), np.zeros((5, 0))
+    q += np.random.default_rng(2).uniform(-0.3, 0.3, q.shape)
+  else:
+    mjm, q, v, u, _ = case(name)
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, u, nconmax=5 * 128, njmax=5 * 512)
+  try:
+    mjw.set_tune(m, d, solver_cta_warps=2, hessian_tc=tc)
+    mjw.forward(m, d)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+      mjw.forward(m, d)
+      torch.cuda.synchronize()
+  finally:
+    mjw.set_tune(m, d, solver_cta_warps=4 if mjm.nv > 128 else 0)
+  assert np.all(mjw.world_status(d) == 0)
+  p.export_chrome_trace(str(tmp_path / "trace.json"))
+  events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+  smem = [e["args"]["shared memory"] for e in events if "k_solve_cta" in e.get("name", "") and "shared memory" in e.get("args", {})]
+  assert smem and max(smem) <= 228 * 1024 // 8 - 1024, smem
