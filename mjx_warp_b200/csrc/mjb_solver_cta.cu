@@ -11,6 +11,6 @@ void launch_solver_cta(const MjbModel* m, const MjbData* d, int nw, int tc, cuda
   else launch_cta<8, false>(m, d, tc, s);
 }
 
-bool solver_cta_takes_warp(const MjbModel* m) { return sparse_launch<1, false>(*m, false); }
+bool solver_cta_takes_warp(const MjbModel* m) { return sparse_launch<1>(*m, false); }
 
 }  // namespace mjb

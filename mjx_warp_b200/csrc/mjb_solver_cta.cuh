@@ -24,6 +24,8 @@
 
 #include "mjb_solver.cuh"
 
+#pragma nv_diag_suppress 20168  // an unroll value of 0 (CtaSolver::kU) leaves a loop without a pragma
+
 namespace mjb {
 
 // CTA sums of K values: warp sums, then the NW warps' partials added in warp order; every thread
@@ -378,9 +380,9 @@ constexpr int kSpFloats = int((sizeof(SH) + 15) / 16 * 4);
 
 // the launches that look for a structure in each world, by the model and the Hessian's assembly; the
 // others keep the dense forms' small part of shared memory
-template <int NW, bool PREC>
+template <int NW>
 __host__ __device__ __forceinline__ bool sparse_launch(const MjbModel& m, bool tc) {
-  return !PREC && !tc && m.nblock >= 2 && m.nblock <= kSpTrees && m.nv <= SparseFor<NW>::kDofs;
+  return !tc && m.nblock >= 2 && m.nblock <= kSpTrees && m.nv <= SparseFor<NW>::kDofs;
 }
 
 __device__ __forceinline__ unsigned long long bits_below(int b) {  // bits 0 .. b - 1
@@ -1293,7 +1295,11 @@ static __device__ __noinline__ void cta_solve_m(const MjbModel& m, const MjbData
   solve_m_world(m, d, w, x, y, lane);
 }
 
-template <int NW, bool PREC>
+// TREES: worlds over nonzero trees and tiles (sparse_launch), the dense routines for those that do not
+// fit; else the dense routines only, in kernels of their own, their loops left to the compiler: kept
+// rolled, as the structure's kernels need them, they have fewer loads in flight (forward of 1024 worlds
+// of a 140-dof chain 19.9 against 17.3 ms, of 2048 worlds of 66 free spheres 35.6 against 33.0).
+template <int NW, bool PREC, bool TREES>
 struct CtaSolver {
   const MjbModel& m;
   const MjbData& d;
@@ -1318,7 +1324,9 @@ struct CtaSolver {
   float qg[3];
   static constexpr int NT = NW * 32;
 
-  __device__ __forceinline__ bool sparse() const { return !PREC && sp; }
+  static constexpr int kU = TREES ? 1 : 0;  // loops that both forms run: rolled, or no pragma
+
+  __device__ __forceinline__ bool sparse() const { return TREES && sp; }
 
   template <int K>
   __device__ __forceinline__ void sum(float (&v)[K]) { cta_sum<NW, K, float>(v, red, warp, lane); }
@@ -1343,12 +1351,12 @@ struct CtaSolver {
   // sparse one's diagonal-plus-ancestor products, one tree per thread
   __device__ void mul_m(float* res, const float* vec) {
     if (m.is_sparse) {
-#pragma unroll 1
+#pragma unroll kU
       for (int blk = tid; blk < m.nblock; blk += NT) {
         const int a = m.block_adr[blk], size = m.block_size[blk];
-#pragma unroll 1
+#pragma unroll kU
         for (int i = a; i < a + size; i++) res[i] = qM[m.dof_Madr[i]] * vec[i];
-#pragma unroll 1
+#pragma unroll kU
         for (int i = a; i < a + size; i++) {
           int Mij = m.dof_Madr[i] + 1;
 #pragma unroll 1
@@ -1361,7 +1369,7 @@ struct CtaSolver {
       __syncthreads();
       return;
     }
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) {
       int a, size;
       if (sparse()) {
@@ -1373,7 +1381,7 @@ struct CtaSolver {
       }
       const float* row = qM + size_t(i) * nv;
       float s = 0.f;
-#pragma unroll 1
+#pragma unroll kU
       for (int j = a; j < a + size; j++) s += row[j] * vec[j];
       res[i] = s;
     }
@@ -1457,11 +1465,11 @@ struct CtaSolver {
       __syncthreads();
       return;
     }
-#pragma unroll 1
+#pragma unroll kU
     for (int k = warp; k < n; k += NW) {
       const float* J = d.efc_J + size_t(adr + k) * nv;
       float v = 0.f;
-#pragma unroll 1
+#pragma unroll kU
       for (int i = lane; i < nv; i += 32) v += J[i] * x[i];
       v = warp_sum(v);
       if (lane == 0) out[adr + k] = sub ? v - sub[adr + k] : v;
@@ -1474,7 +1482,7 @@ struct CtaSolver {
     prev_cost = cost;
     float c[2] = {0.f, 0.f};
     bool ch = false;
-#pragma unroll 1
+#pragma unroll kU
     for (int k = tid; k < n; k += NT) {
       const int r = adr + k;
       const float Jaref = d.efc_Jaref[r], D = d.efc_D[r];
@@ -1493,7 +1501,7 @@ struct CtaSolver {
       }
     }
     changed = __syncthreads_or(ch) != 0;
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) {
       float f = 0.f;
       if (sparse()) {
@@ -1505,7 +1513,7 @@ struct CtaSolver {
           if (fk != 0.f) f += row_entries(k, t)[i - a] * fk;
         }
       }
-#pragma unroll 1
+#pragma unroll kU
       for (int k = sparse() ? n : 0; k < n; k++) {
         const float fk = d.efc_force[adr + k];
         if (fk != 0.f) f += d.efc_J[size_t(adr + k) * nv + i] * fk;
@@ -1761,7 +1769,7 @@ struct CtaSolver {
   // solver.py:176-312
   __device__ void update_gradient() {
     float gd[1] = {0.f};
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) {
       const float g = Ma[i] - qfrc_smooth[i] - qfrc_constraint[i];
       grad[i] = g;
@@ -1778,7 +1786,7 @@ struct CtaSolver {
       if (PREC) {  // H in split TF32 straight into the FP64 tile, factored there in FP64
         assemble_hessian_tc<double, true>(Ld, 0);
         chol_cta_d<NW>(Ld, rdg, nv, warp, lane);
-#pragma unroll 1
+#pragma unroll kU
         for (int e = tid; e < nv * nv; e += NT) {  // efc_h keeps the factor (FP32-rounded)
           const int i = e / nv, j = e - i * nv;
           if (j <= i) H[e] = float(Ld[tri(i) + j]);
@@ -1788,7 +1796,7 @@ struct CtaSolver {
           assemble_hessian_sparse();
           chol_cta_sparse<NW, SH>(nv, T, *S, warp, lane);
         } else if constexpr (NW > 1) {
-          if (tc) assemble_hessian_tc(H, nv);
+          if (!TREES && tc) assemble_hessian_tc(H, nv);
           else assemble_hessian();
           chol_cta<NW>(H, nv, nv, T, warp, lane);
         }
@@ -1831,7 +1839,7 @@ struct CtaSolver {
     mul_m(mv, search);
     {
       float q[3] = {0.f, 0.f, 0.f};
-#pragma unroll 1
+#pragma unroll kU
       for (int i = tid; i < nv; i += NT) {
         q[0] += gauss / float(nv);
         q[1] += search[i] * (Ma[i] - qfrc_smooth[i]);
@@ -1848,7 +1856,7 @@ struct CtaSolver {
     constexpr int kRegRows = 3;
     const bool regs = n <= kRegRows * NT;
     float rJ[kRegRows], rv[kRegRows], rq[kRegRows][3];
-#pragma unroll 1
+#pragma unroll kU
     for (int k = tid, e = 0; k < n; k += NT, e++) {
       const int r = adr + k;
       const float jv = d.efc_jv[r], Jaref = d.efc_Jaref[r], D = d.efc_D[r];
@@ -1873,7 +1881,7 @@ struct CtaSolver {
         for (int h = 0; h < kRegRows; h++)
           if (tid + h * NT < n) f(rJ[h], rv[h], rq[h]);
       } else {
-#pragma unroll 1
+#pragma unroll kU
         for (int k = tid; k < n; k += NT) {
           const int r = adr + k;
           f(d.efc_Jaref[r], d.efc_jv[r], d.efc_quad + 3 * r);
@@ -2005,12 +2013,12 @@ struct CtaSolver {
       }
     }
     // solver.py:816-841
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) {
       qacc[i] += alpha * search[i];
       Ma[i] += alpha * mv[i];
     }
-#pragma unroll 1
+#pragma unroll kU
     for (int k = tid; k < n; k += NT) d.efc_Jaref[adr + k] += alpha * d.efc_jv[adr + k];
     __syncthreads();
   }
@@ -2018,7 +2026,7 @@ struct CtaSolver {
   // search = -Mgrad (+ beta search for CG); returns search . search
   __device__ void new_search() {
     float sd[1] = {0.f};
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) {
       float v = -Mgrad[i];
       if (m.solver == 1) v += beta * search[i];
@@ -2037,9 +2045,9 @@ struct CtaSolver {
         solve_generic(m, d, w, lane, H, nz, true);
         return;
       }
-    } else if (sparse_launch<NW, PREC>(m, tc))
+    } else if constexpr (TREES)
       sp = sparse_shape<NW, SH>(m, d.efc_J + size_t(adr) * nv, n, H, *S, cw, warp, lane);
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) qacc[i] = ws[i];
     __syncthreads();
     // _create_context (solver.py:26-72)
@@ -2059,7 +2067,7 @@ struct CtaSolver {
       if (it >= 0) {
         linesearch();
         if (m.solver == 1) {
-#pragma unroll 1
+#pragma unroll kU
           for (int i = tid; i < nv; i += NT) {
             prev_grad[i] = grad[i];
             prev_Mgrad[i] = Mgrad[i];
@@ -2071,7 +2079,7 @@ struct CtaSolver {
       update_gradient();
       if (it >= 0 && m.solver == 1) {  // Polak-Ribiere (solver.py:918-970)
         float nd[2] = {0.f, 0.f};
-#pragma unroll 1
+#pragma unroll kU
         for (int i = tid; i < nv; i += NT) {
           nd[0] += grad[i] * (Mgrad[i] - prev_Mgrad[i]);
           nd[1] += prev_grad[i] * prev_Mgrad[i];
@@ -2085,7 +2093,7 @@ struct CtaSolver {
     }
     if (sparse() && factored && S->L != H) store_factor();
     float* wsw = d.qacc_warmstart + W(w, nv);
-#pragma unroll 1
+#pragma unroll kU
     for (int i = tid; i < nv; i += NT) wsw[i] = qacc[i];
     if (tid == 0) {
       if (d.efc_cost) d.efc_cost[w] = cost;
@@ -2108,12 +2116,12 @@ struct CtaSolver {
   }
 };
 
-// One world's solve by the whole CTA; smem: cta_solver_smem_floats(nv, NW, PREC, sparse_launch) floats
-template <int NW, bool PREC>
+// One world's solve by the whole CTA; smem: cta_solver_smem_floats(nv, NW, PREC, TREES) floats
+template <int NW, bool PREC, bool TREES>
 __device__ void solve_cta(const MjbModel& m, const MjbData& d, int w, float* smem, bool tc) {
   const int nv = m.nv;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  CtaSolver<NW, PREC> s{m, d, w, tid, lane, warp, nv, d.world_efcadr[w], d.world_nefc[w]};
+  CtaSolver<NW, PREC, TREES> s{m, d, w, tid, lane, warp, nv, d.world_efcadr[w], d.world_nefc[w]};
   s.qacc = d.qacc + W(w, nv);
   s.Ma = d.efc_Ma + W(w, nv);
   s.grad = d.efc_grad + W(w, nv);
