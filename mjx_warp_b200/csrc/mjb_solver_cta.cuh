@@ -2040,6 +2040,7 @@ struct CtaSolver {
   __device__ void run() {
     const float* ws = d.qacc_warmstart + W(w, nv);
     if constexpr (NW == 1) {  // solve_generic's arithmetic, which takes the worlds that do not fit
+      if (n > SH::kRows) return;  // k_solve_many_rows's
       sp = sparse_shape<NW, SH>(m, d.efc_J + size_t(adr) * nv, n, H, *S, cw, warp, lane);
       if (!sp) {
         solve_generic(m, d, w, lane, H, nz, true);

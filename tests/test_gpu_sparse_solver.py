@@ -191,3 +191,36 @@ def test_dense_launches_keep_their_shared_memory(name, tc, tmp_path):
   events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
   smem = [e["args"]["shared memory"] for e in events if "k_solve_cta" in e.get("name", "") and "shared memory" in e.get("args", {})]
   assert smem and max(smem) <= 228 * 1024 // 8 - 1024, smem
+
+
+@pytest.mark.parametrize("ordered", [True, False])
+def test_one_warp_worlds_past_the_row_capacity(ordered):
+  """Worlds of 0 to 320 rows (boxes on a plane, 4 contacts each) mixed in one batch, more and fewer than the
+  192 rows of the one-warp structure: every world is solved, once, to the plain form's values, with the
+  work queue and without."""
+  boxes = "".join(f'<body pos="{0.5 * (i % 5)} {0.5 * (i // 5)} 0.058"><freejoint/>'
+                  '<geom type="box" size="0.1 0.08 0.06"/></body>' for i in range(20))
+  mjm = load('<mujoco><option timestep="0.002"/><worldbody><geom type="plane" size="0 0 1"/>' + boxes
+             + "</worldbody></mujoco>", iterations=5, ls_iterations=10, jacobian=MJ_JAC_DENSE)
+  nworld, rng = 37, np.random.default_rng(4)
+  q = np.tile(mjm.qpos0, (nworld, 1))
+  x = q.reshape(nworld, 20, 7)
+  x[:, :, :2] += rng.uniform(-0.05, 0.05, (nworld, 20, 2))
+  for w in range(nworld):
+    x[w, w % 21:, 2] += 1.0  # w mod 21 boxes touch the plane
+  v = rng.normal(0.0, 0.1, (nworld, mjm.nv))
+  m = mjw.put_model(mjm)
+  out = {}
+  for form in (1, 0):
+    d = device_data(mjm, q, v, np.zeros((nworld, 0)), nconmax=100 * nworld, njmax=400 * nworld)
+    if not ordered:
+      d.work_queue = None
+    mjw.forward(m, d, fused=form)
+    torch.cuda.synchronize()
+    assert np.all(mjw.world_status(d) == 0)
+    out[form] = d
+  n = world_rows(out[1], "efc")[0]
+  assert n.min() == 0 and n.max() == 320 and np.any(n == 192) and np.any(n == 208)
+  for f in ("qacc", "qfrc_constraint", "qacc_warmstart"):
+    assert torch.equal(getattr(out[1], f), getattr(out[0], f)), f
+  assert torch.equal(out[1].efc.h.tril(), out[0].efc.h.tril())
