@@ -55,7 +55,7 @@ enum Stage {
 // make_constraint's lanes hold a contact each and need 80 registers (6 CTAs per SM: the fastest of
 // 5, 6 and 8 on 8192 and on 32768 humanoid worlds, by 1 %); every other stage is held to 64 for
 // occupancy
-template <int STAGE>
+template <int STAGE, bool PACK>
 __global__ void __launch_bounds__(128, STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB_STAGE)
     k_stage(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int smem_per_warp) {
   extern __shared__ __align__(16) float smem[];
@@ -67,20 +67,20 @@ __global__ void __launch_bounds__(128, STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB
     case S_KINEMATICS: kinematics(m, d, w, lane); break;
     case S_COM_POS: com_pos(m, d, w, lane); break;
     case S_CRB: crb(m, d, w, lane); break;
-    case S_FACTOR_M: factor_m(m, d, w, lane, sm); break;
+    case S_FACTOR_M: factor_m<PACK>(m, d, w, lane, sm); break;
     case S_TRANSMISSION: transmission(m, d, w, lane); break;
     case S_COM_VEL: com_vel(m, d, w, lane); break;
     case S_PASSIVE: passive(m, d, w, lane); break;
     case S_RNE: rne(m, d, w, lane); break;
     case S_FWD_VELOCITY: fwd_velocity(m, d, w, lane); break;
     case S_FWD_ACTUATION: fwd_actuation(m, d, w, lane); break;
-    case S_FWD_ACCELERATION: fwd_acceleration(m, d, w, lane, sm); break;
+    case S_FWD_ACCELERATION: fwd_acceleration<PACK>(m, d, w, lane, sm); break;
     case S_NXN: nxn_broadphase(m, d, w, lane); break;
     case S_SAP: sap_broadphase(m, d, w, lane, sm); break;
     case S_NARROW: primitive_narrowphase(m, d, w, lane); break;
     case S_MAKE_CONSTRAINT: make_constraint(m, d, w, lane); break;
-    case S_EULER: euler(m, d, w, lane, sm); break;
-    case S_IMPLICIT: implicit(m, d, w, lane, sm); break;
+    case S_EULER: euler<PACK>(m, d, w, lane, sm); break;
+    case S_IMPLICIT: implicit<PACK>(m, d, w, lane, sm); break;
     case S_QACC_SMOOTH_COPY: copy_qacc_smooth(m, d, w, lane); break;
     case S_CHECK: check_finite(m, d, w, lane); break;
   }
@@ -183,14 +183,15 @@ __global__ void __launch_bounds__(1024) k_order_worlds(const int* nefc, int* ord
 }
 
 // chosen form: integration (forward.py:165-405) and the finiteness check
+template <bool PACK>
 __global__ void __launch_bounds__(128, MJB_MINB_INT) k_integrate(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int tile_per_warp) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= d.nworld) return;
   float* tile = smem + size_t(threadIdx.x >> 5) * tile_per_warp;
-  if (m.integrator == 0) euler(m, d, w, lane, tile);
-  else implicit(m, d, w, lane, tile);
+  if (m.integrator == 0) euler<PACK>(m, d, w, lane, tile);
+  else implicit<PACK>(m, d, w, lane, tile);
   check_finite(m, d, w, lane);
 }
 
@@ -491,26 +492,35 @@ int fused_smem_per_warp(const MjbModel* m) {
 }
 
 
+// the stages that factor or solve tree blocks are compiled twice (PACK, mjb_world.cuh)
+constexpr bool packs(int stage) {
+  return stage == S_FACTOR_M || stage == S_FWD_ACCELERATION || stage == S_EULER || stage == S_IMPLICIT;
+}
+inline bool packed(const MjbModel* m) { return m->nblock > 1; }
+
+template <int STAGE, bool PACK>
+int launch_stage_form(const MjbModel* m, const MjbData* d, int spw, cudaStream_t s) {
+  const size_t bytes = size_t(spw) * kDefaultWarps * sizeof(float);
+  if (bytes > kMaxSmemPerCta) return MJB_ERR_SCRATCH;
+  static size_t configured[kSmemDevices];
+  allow_smem(k_stage<STAGE, PACK>, bytes, configured);
+  k_stage<STAGE, PACK><<<grid_for(d->nworld, kDefaultWarps), 32 * kDefaultWarps, bytes, s>>>(*m, *d, spw);
+  return finish();
+}
+
 template <int STAGE>
 int launch_stage(const MjbModel* m, const MjbData* d, cudaStream_t s) {
   if (int rc = stage_fields(STAGE, m, d)) return rc;
   if constexpr (STAGE == S_SOLVE) {
     return launch_solver_plain(m, d, s);
   } else {
-    const int warps = kDefaultWarps;
     int spw = 0;
-    size_t bytes = 0;
-    if (STAGE == S_FACTOR_M || STAGE == S_FWD_ACCELERATION || STAGE == S_EULER || STAGE == S_IMPLICIT)
-      spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
+    if (packs(STAGE)) spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
     if (STAGE == S_SAP) spw = sap_smem_floats(m->ngeom);
-    if (spw) {
-      bytes = size_t(spw) * warps * sizeof(float);
-      if (bytes > kMaxSmemPerCta) return MJB_ERR_SCRATCH;
-      static size_t configured[kSmemDevices];
-      allow_smem(k_stage<STAGE>, bytes, configured);
+    if constexpr (packs(STAGE)) {
+      if (packed(m)) return launch_stage_form<STAGE, true>(m, d, spw, s);
     }
-    k_stage<STAGE><<<grid_for(d->nworld, warps), 32 * warps, bytes, s>>>(*m, *d, spw);
-    return finish();
+    return launch_stage_form<STAGE, false>(m, d, spw, s);
   }
 }
 
@@ -773,7 +783,6 @@ int run_chosen_phase(const MjbModel* m, const MjbData* d, int phase, cudaStream_
   const int grid = grid_for(d->nworld, warps);
   const int tpw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
   const size_t tile_bytes = size_t(tpw) * warps * sizeof(float);
-  static size_t conf_int[kSmemDevices];
   if (phase == 0) {
     reset_counters(d, true, true, true, true, s);
     int rc = run_forward_fork(m, d, s, cfg.lanes);
@@ -787,8 +796,10 @@ int run_chosen_phase(const MjbModel* m, const MjbData* d, int phase, cudaStream_
       else launch_solver<false>(m, d, cfg, spw, s);
     }
   } else if (phase == 2) {
-    allow_smem(k_integrate, tile_bytes, conf_int);
-    k_integrate<<<grid, 32 * warps, tile_bytes, s>>>(*m, *d, tpw);
+    static size_t conf_int[2][kSmemDevices];
+    const auto k = packed(m) ? k_integrate<true> : k_integrate<false>;
+    allow_smem(k, tile_bytes, conf_int[packed(m)]);
+    k<<<grid, 32 * warps, tile_bytes, s>>>(*m, *d, tpw);
   } else {
     return MJB_ERR_ARG;
   }

@@ -782,6 +782,10 @@ static __device__ __noinline__ void chol_tile_d_groups(double* A, int ld, int n,
 // its own first column in either place, so the factor is that of the block by itself.  One block at
 // a time left the warp waiting out 64 short chains per world of the bin (384 dofs) and 17 of the
 // humanoid with spheres.
+//
+// PACK, of the routines below: compiled for models of several blocks.  The host picks the stage kernels by
+// nblock; the kernels of one block do without the packed code, which took registers that they spilled
+// (fwd_acceleration in the precision form, 8192 humanoid worlds: 108 us with it, 70 without).
 struct BlockPack {
   int cnt;         // blocks, 0 or 1: not packed
   int a, n;        // this lane's block: first dof and size (0: none)
@@ -972,6 +976,7 @@ static __device__ void warp_cho_solve(const float* L, int ld, int n, float* x, c
 // into L (smooth.py:353-379, qLD_tile semantics; zeros outside the blocks' lower triangles).  With
 // a per-warp tile, blocks of n <= 32 are factored in shared memory and written back row by row;
 // the tile then holds the factor of the last block.
+template <bool PACK = true>
 static __device__ void factor_blocks(const MjbModel& m, const float* M, float* L, int lane,
                               const float* dadd = nullptr, float scale = 0.f, float* tile = nullptr) {
   const int nv = m.nv;
@@ -981,7 +986,7 @@ static __device__ void factor_blocks(const MjbModel& m, const float* M, float* L
     __syncwarp();
   }
   for (int blk = 0; blk < m.nblock; blk++) {
-    if (tile && nv >= 32) {  // a tile of 32 rows
+    if (PACK && tile && nv >= 32) {  // a tile of 32 rows
       const BlockPack p = pack_blocks(m, blk, lane);
       if (p.cnt > 1) {
         const int tld = tile_ld(nv), c = lane & 7, at = (lane & 24) * tld + lane;
@@ -1037,11 +1042,12 @@ static __device__ void factor_blocks(const MjbModel& m, const float* M, float* L
 // x = M^-1 y per tree block from the block factor L (smooth.py:654-681); x may alias y.  With a
 // tile, blocks of n <= 32 are staged into it row by row first, unless tile_has_factor says that
 // the tile already holds the factor of the model's only block.
+template <bool PACK = true>
 static __device__ void solve_blocks(const MjbModel& m, const float* L, float* x, const float* y,
                              int lane, float* tile = nullptr, bool tile_has_factor = false) {
   const int nv = m.nv;
   for (int blk = 0; blk < m.nblock; blk++) {
-    if (m.nblock > 1) {
+    if (PACK && m.nblock > 1) {
       const BlockPack p = pack_blocks(m, blk, lane);
       if (p.cnt > 1) {
         const int c = lane & 7;
@@ -1087,11 +1093,12 @@ static __device__ void solve_blocks(const MjbModel& m, const float* L, float* x,
 
 // x = (M + scale diag(dadd))^-1 y per tree block, factored and solved in FP64 in the double tile
 // dt (precision form; blocks of n <= 32, dense M with leading dimension nv).
+template <bool PACK = true>
 static __device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, const float* dadd,
                                       float scale, float* x, const float* y, int lane, double* dt) {
   const int nv = m.nv, ld = tile_ld(nv);
   for (int blk = 0; blk < m.nblock; blk++) {
-    if (nv >= 32) {
+    if (PACK && nv >= 32) {
       const BlockPack p = pack_blocks(m, blk, lane);
       if (p.cnt > 1) {
         const int c = lane & 7, at = (lane & 24) * ld + lane;
@@ -1132,6 +1139,7 @@ static __device__ void factor_solve_blocks_d(const MjbModel& m, const float* M, 
 }
 
 // smooth.py:392-395
+template <bool PACK = true>
 static __device__ void factor_m(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv;
   if (m.is_sparse) {  // smooth.py:317-351
@@ -1142,15 +1150,16 @@ static __device__ void factor_m(const MjbModel& m, const MjbData& d, int w, int 
     factor_sparse(m, L, d.qLDiagInv + W(w, nv), lane);
     return;
   }
-  factor_blocks(m, d.qM + W(w, nv * nv), d.qLD + W(w, nv * nv), lane, nullptr, 0.f, tile);
+  factor_blocks<PACK>(m, d.qM + W(w, nv * nv), d.qLD + W(w, nv * nv), lane, nullptr, 0.f, tile);
 }
 
 // x = M^-1 y with the world's mass-matrix factor (qLD), dense or sparse
+template <bool PACK = true>
 __device__ __forceinline__ void solve_m_world(const MjbModel& m, const MjbData& d, int w, float* x,
                                               const float* y, int lane, float* tile = nullptr,
                                               bool tile_has_factor = false) {
   if (m.is_sparse) solve_sparse(m, d.qLD + W(w, m.nM), d.qLDiagInv + W(w, m.nv), x, y, lane);
-  else solve_blocks(m, d.qLD + W(w, m.nv * m.nv), x, y, lane, tile, tile_has_factor);
+  else solve_blocks<PACK>(m, d.qLD + W(w, m.nv * m.nv), x, y, lane, tile, tile_has_factor);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1429,6 +1438,7 @@ static __device__ void xfrc_accumulate(const MjbModel& m, const MjbData& d, int 
 
 // forward.py:644-661
 // tile_has_qLD: the per-warp tile still holds the factor left by factor_m
+template <bool PACK = true>
 static __device__ void fwd_acceleration(const MjbModel& m, const MjbData& d, int w, int lane,
                                  float* tile = nullptr, bool tile_has_qLD = false) {
   const int nv = m.nv;
@@ -1441,11 +1451,11 @@ static __device__ void fwd_acceleration(const MjbModel& m, const MjbData& d, int
   __syncwarp();
   xfrc_accumulate(m, d, w, sm, lane);
   if (m.precision && tile) {  // FP64 factor-solve in the double tile after the float tile
-    factor_solve_blocks_d(m, d.qM + W(w, nv * nv), nullptr, 0.f, d.qacc_smooth + W(w, nv), sm, lane,
+    factor_solve_blocks_d<PACK>(m, d.qM + W(w, nv * nv), nullptr, 0.f, d.qacc_smooth + W(w, nv), sm, lane,
                           reinterpret_cast<double*>(tile + tile_floats(nv)));
     return;
   }
-  solve_m_world(m, d, w, d.qacc_smooth + W(w, nv), sm, lane, tile, tile_has_qLD);
+  solve_m_world<PACK>(m, d, w, d.qacc_smooth + W(w, nv), sm, lane, tile, tile_has_qLD);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1472,6 +1482,7 @@ static __device__ void advance(const MjbModel& m, const MjbData& d, int w, const
 }
 
 // forward.py:165-242 — Euler with implicit joint damping unless EULERDAMP is disabled
+template <bool PACK = true>
 static __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv;
   if (m.disableflags & DSBL_EULERDAMP) {
@@ -1505,19 +1516,20 @@ static __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lan
     return;
   }
   float* L = d.qLD_integration + W(w, nv * nv);
-  factor_blocks(m, d.qM + W(w, nv * nv), L, lane, m.dof_damping, m.timestep, tile);
+  factor_blocks<PACK>(m, d.qM + W(w, nv * nv), L, lane, m.dof_damping, m.timestep, tile);
   for (int i = lane; i < nv; i += 32) x[i] = sm[i] + qc[i];
   __syncwarp();
   if (m.precision && tile)  // the float factor stays in qLD_integration; x in FP64
-    factor_solve_blocks_d(m, d.qM + W(w, nv * nv), m.dof_damping, m.timestep, x, x, lane,
+    factor_solve_blocks_d<PACK>(m, d.qM + W(w, nv * nv), m.dof_damping, m.timestep, x, x, lane,
                           reinterpret_cast<double*>(tile + tile_floats(nv)));
   else
-    solve_blocks(m, L, x, x, lane, tile, true);
+    solve_blocks<PACK>(m, L, x, x, lane, tile, true);
   advance(m, d, w, x, lane);
 }
 
 // forward.py:245-405 — implicitfast (dense): (M - dt qDeriv) qacc = qfrc_smooth + qfrc_constraint
 // with qDeriv = moment^T diag(bias_vel + gain_vel * ctrl) moment - diag(damping)
+template <bool PACK = true>
 static __device__ void implicit(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv, nu = m.nu;
   const bool passive_on = !(m.disableflags & DSBL_PASSIVE);
@@ -1590,11 +1602,11 @@ static __device__ void implicit(const MjbModel& m, const MjbData& d, int w, int 
     }
   }
   if (!tiled) {
-    factor_blocks(m, Mi, L, lane, nullptr, 0.f, tile);
-    solve_blocks(m, L, x, f, lane);
+    factor_blocks<PACK>(m, Mi, L, lane, nullptr, 0.f, tile);
+    solve_blocks<PACK>(m, L, x, f, lane);
   }
   if (m.precision && tile)  // the float factor stays in qLD_integration; x again in FP64
-    factor_solve_blocks_d(m, Mi, nullptr, 0.f, x, f, lane,
+    factor_solve_blocks_d<PACK>(m, Mi, nullptr, 0.f, x, f, lane,
                           reinterpret_cast<double*>(tile + tile_floats(nv)));
   advance(m, d, w, x, lane);
 }
