@@ -1289,6 +1289,16 @@ static __device__ __noinline__ void cho_solve_d_regs(const double* P, const doub
   __syncwarp();
 }
 
+// A gradient with a NaN or an infinity in it (grad_dot alone may overflow): the dense substitution
+// multiplies it with the zeros between the trees, so that every entry becomes NaN.  So it does here: no
+// tree of a world that has gone wrong looks solved.
+static __device__ __noinline__ void spread_nonfinite(const float* grad, float* Mgrad, int nv, int tid, int nt) {
+  bool bad = false;
+  for (int i = tid; i < nv; i += nt) bad |= !isfinite(grad[i]);
+  if (!__syncthreads_or(bad)) return;
+  for (int i = tid; i < nv; i += nt) Mgrad[i] = __int_as_float(0x7fffffff);
+}
+
 // the CG preconditioner, kept out of the Newton solver's code
 static __device__ __noinline__ void cta_solve_m(const MjbModel& m, const MjbData& d, int w, float* x,
                                                 const float* y, int lane) {
@@ -1807,8 +1817,10 @@ struct CtaSolver {
       if (PREC && nv <= 128) cho_solve_d_regs(Ld, rdg, nv, Mgrad, grad, lane);
       else if (PREC) cho_solve_d_warp(Ld, rdg, nv, vd, Mgrad, grad, lane);
     }
-    if (sparse()) cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
-    else if constexpr (!PREC && NW > 1) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
+    if (sparse()) {
+      cho_solve_cta_sparse<NW, SH>(nv, Mgrad, grad, zv, *S, warp, lane);
+      if (!isfinite(grad_dot)) spread_nonfinite(grad, Mgrad, nv, tid, NT);
+    } else if constexpr (!PREC && NW > 1) cho_solve_cta<NW>(H, nv, nv, Mgrad, grad, zv, red, warp, lane);
     __syncthreads();
   }
 

@@ -224,3 +224,26 @@ def test_one_warp_worlds_past_the_row_capacity(ordered):
   for f in ("qacc", "qfrc_constraint", "qacc_warmstart"):
     assert torch.equal(getattr(out[1], f), getattr(out[0], f)), f
   assert torch.equal(out[1].efc.h.tril(), out[0].efc.h.tril())
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("name", ["spheres6", "spheres11", "bin"])
+def test_nonfinite_force_reaches_every_tree(name, bad):
+  """A NaN or an infinite force on one dof of one tree: the world's accelerations are not finite where the
+  plain form's are not (its dense solve multiplies them with the zeros between the trees), and the
+  other worlds are what they are without it."""
+  mjm, q, v, u, cap = case(name)
+  mjm.opt.iterations = 5
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  qacc = {}
+  for key, form, force in (("clean", 1, 0.0), ("chosen", 1, bad), ("plain", 0, bad)):
+    d = device_data(mjm, q, v, u, nconmax=800 * nworld, njmax=cap * nworld)
+    d.qfrc_applied[1, 8] = force
+    mjw.forward(m, d, fused=form)
+    torch.cuda.synchronize()
+    qacc[key] = dev(d.qacc)
+  plain = np.isfinite(qacc["plain"])
+  assert not plain[1].any() and np.delete(plain, 1, axis=0).all()
+  assert np.array_equal(np.isfinite(qacc["chosen"]), plain)
+  assert np.array_equal(np.delete(qacc["chosen"], 1, axis=0), np.delete(qacc["clean"], 1, axis=0))
