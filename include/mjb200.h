@@ -178,9 +178,10 @@ typedef struct MjbStepIO {
   float *qpos_out, *qvel_out, *qacc_warmstart_out, *xpos_out, *xmat_out, *subtree_com_out,
       *cvel_out, *site_xpos_out;
 } MjbStepIO;
-/* Copy in, nstep calls of mjb_step (cfg as there), copy out: every copy is one
- * cudaMemcpyAsync on the stream, so the call allocates nothing, does not synchronise and can be
- * captured in a CUDA graph; no counterpart function in the reference, whose callers write these
+/* Copy in, nstep calls of mjb_step (cfg as there), copy out: the copies each way are one kernel on
+ * the stream (a cudaMemcpyAsync for a buffer that is not this device's; pageable host memory is
+ * refused), so the call allocates nothing, does not synchronise and can be captured in a CUDA graph;
+ * no counterpart function in the reference, whose callers write these
  * copies around step themselves. */
 int mjb_step_io(const MjbModel* m, const MjbData* d, const MjbStepIO* io, int nstep,
                 const MjbRunCfg* cfg, mjbStream stream);

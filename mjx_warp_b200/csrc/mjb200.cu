@@ -728,8 +728,9 @@ struct Copy {
   size_t bytes;
 };
 // The requested ones of n <= 8 copies: one k_copy for those between buffers of this device, a
-// cudaMemcpyAsync for any other (pinned host memory, another device's), and one for each, in order,
-// when a copy's destination overlaps another's buffers.
+// device-to-device cudaMemcpyAsync for any other (another device's, pinned host memory; pageable host
+// memory is refused: a copy of it would wait for the host), and one for each, in order, when a copy's
+// destination overlaps another's buffers.
 int copy_all(const Copy* c, int n, cudaStream_t s) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return MJB_ERR_LAUNCH;
@@ -762,7 +763,7 @@ int copy_all(const Copy* c, int n, cudaStream_t s) {
       l.dst[k] = static_cast<uint32_t*>(c[i].dst);
       l.n[k] = c[i].bytes / 4;
       most = std::max(most, l.n[k++]);
-    } else if (cudaMemcpyAsync(c[i].dst, c[i].src, c[i].bytes, cudaMemcpyDefault, s) != cudaSuccess) {
+    } else if (cudaMemcpyAsync(c[i].dst, c[i].src, c[i].bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
       return MJB_ERR_LAUNCH;
     }
   }

@@ -2,11 +2,14 @@
 staged capacity, tree blocks packed four to a tile, constraint rows past eight contacts, and the
 one-launch copies of step_io."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import mjx_warp_b200 as mjw
+from mjx_warp_b200 import _abi
 from mjx_warp_b200.types import MJ_JAC_DENSE
 from helpers import dev, device_data, humanoid, humanoid_state, load, oracle, world_rows
 from test_gpu_configs import bin_state, humanoid_spheres_state
@@ -220,3 +223,27 @@ def test_step_io_overlapping_buffers_keep_their_order():
   mjw.step_io(m, want, 1, outputs=())
   torch.cuda.synchronize()
   assert torch.equal(d.qvel, want.qvel)
+
+
+@pytest.mark.parametrize("field", ["qpos", "qpos_out"])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_step_io_host_buffers(field, pinned):
+  """The C entry takes pinned host buffers and refuses pageable ones (a copy of those would wait for the
+  host).  Under capture, so nothing runs."""
+  mjm = humanoid()
+  q, v, u = humanoid_state(mjm, 4, seed=1)
+  m = mjw.put_model(mjm)
+  d = device_data(mjm, q, v, u)
+  mjw.step(m, d)  # the forked streams exist before the capture
+  torch.cuda.synchronize()
+  host = torch.zeros(q.shape, dtype=torch.float32, pin_memory=pinned)
+  io = _abi.MjbStepIO()
+  setattr(io, field, host.data_ptr())
+  g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+  with torch.cuda.stream(s):
+    g.capture_begin(capture_error_mode="thread_local")
+    rc = _abi.lib().mjb_step_io(ctypes.byref(_abi.model_view(m)), ctypes.byref(_abi.data_view(d)),
+                                ctypes.byref(io), 1, None, s.cuda_stream)
+    g.capture_end()
+  _abi.lib().mjb_error_string(rc)  # takes the error back
+  assert rc == (0 if pinned else 3)  # MJB_ERR_LAUNCH
