@@ -79,8 +79,8 @@ __global__ void __launch_bounds__(128, STAGE == S_MAKE_CONSTRAINT ? 6 : MJB_MINB
     case S_SAP: sap_broadphase(m, d, w, lane, sm); break;
     case S_NARROW: primitive_narrowphase(m, d, w, lane); break;
     case S_MAKE_CONSTRAINT: make_constraint(m, d, w, lane); break;
-    case S_EULER: euler<PACK>(m, d, w, lane, sm); break;
-    case S_IMPLICIT: implicit<PACK>(m, d, w, lane, sm); break;
+    case S_EULER: euler(m, d, w, lane, sm); break;
+    case S_IMPLICIT: implicit(m, d, w, lane, sm); break;
     case S_QACC_SMOOTH_COPY: copy_qacc_smooth(m, d, w, lane); break;
     case S_CHECK: check_finite(m, d, w, lane); break;
   }
@@ -183,15 +183,14 @@ __global__ void __launch_bounds__(1024) k_order_worlds(const int* nefc, int* ord
 }
 
 // chosen form: integration (forward.py:165-405) and the finiteness check
-template <bool PACK>
 __global__ void __launch_bounds__(128, MJB_MINB_INT) k_integrate(const __grid_constant__ MjbModel m, const __grid_constant__ MjbData d, int tile_per_warp) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= d.nworld) return;
   float* tile = smem + size_t(threadIdx.x >> 5) * tile_per_warp;
-  if (m.integrator == 0) euler<PACK>(m, d, w, lane, tile);
-  else implicit<PACK>(m, d, w, lane, tile);
+  if (m.integrator == 0) euler(m, d, w, lane, tile);
+  else implicit(m, d, w, lane, tile);
   check_finite(m, d, w, lane);
 }
 
@@ -492,11 +491,8 @@ int fused_smem_per_warp(const MjbModel* m) {
 }
 
 
-// the stages that factor or solve tree blocks are compiled twice (PACK, mjb_world.cuh)
-constexpr bool packs(int stage) {
-  return stage == S_FACTOR_M || stage == S_FWD_ACCELERATION || stage == S_EULER || stage == S_IMPLICIT;
-}
-inline bool packed(const MjbModel* m) { return m->nblock > 1; }
+// the stages that factor and solve M's tree blocks are compiled twice (PACK, mjb_world.cuh)
+constexpr bool packs(int stage) { return stage == S_FACTOR_M || stage == S_FWD_ACCELERATION; }
 
 template <int STAGE, bool PACK>
 int launch_stage_form(const MjbModel* m, const MjbData* d, int spw, cudaStream_t s) {
@@ -515,10 +511,11 @@ int launch_stage(const MjbModel* m, const MjbData* d, cudaStream_t s) {
     return launch_solver_plain(m, d, s);
   } else {
     int spw = 0;
-    if (packs(STAGE)) spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
+    if (packs(STAGE) || STAGE == S_EULER || STAGE == S_IMPLICIT)
+      spw = tile_floats(m->nv) + (m->precision ? prec_tile_floats(m->nv) : 0);
     if (STAGE == S_SAP) spw = sap_smem_floats(m->ngeom);
     if constexpr (packs(STAGE)) {
-      if (packed(m)) return launch_stage_form<STAGE, true>(m, d, spw, s);
+      if (m->nblock > 1) return launch_stage_form<STAGE, true>(m, d, spw, s);
     }
     return launch_stage_form<STAGE, false>(m, d, spw, s);
   }
@@ -797,10 +794,9 @@ int run_chosen_phase(const MjbModel* m, const MjbData* d, int phase, cudaStream_
       else launch_solver<false>(m, d, cfg, spw, s);
     }
   } else if (phase == 2) {
-    static size_t conf_int[2][kSmemDevices];
-    const auto k = packed(m) ? k_integrate<true> : k_integrate<false>;
-    allow_smem(k, tile_bytes, conf_int[packed(m)]);
-    k<<<grid, 32 * warps, tile_bytes, s>>>(*m, *d, tpw);
+    static size_t conf_int[kSmemDevices];
+    allow_smem(k_integrate, tile_bytes, conf_int);
+    k_integrate<<<grid, 32 * warps, tile_bytes, s>>>(*m, *d, tpw);
   } else {
     return MJB_ERR_ARG;
   }

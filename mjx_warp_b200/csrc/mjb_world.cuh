@@ -783,9 +783,10 @@ static __device__ __noinline__ void chol_tile_d_groups(double* A, int ld, int n,
 // a time left the warp waiting out 64 short chains per world of the bin (384 dofs) and 17 of the
 // humanoid with spheres.
 //
-// PACK, of the routines below: compiled for models of several blocks.  The host picks the stage kernels by
-// nblock; the kernels of one block do without the packed code, which took registers that they spilled
-// (fwd_acceleration in the precision form, 8192 humanoid worlds: 108 us with it, 70 without).
+// PACK, of the routines below: compiled for models of several blocks.  The host picks factor_m's and
+// fwd_acceleration's kernel by nblock; that of one block does without the packed code, which took
+// registers that it spilled (fwd_acceleration in the precision form, 8192 humanoid worlds: 109 us with
+// it, 70 without).  The integrators keep it: without it k_integrate measured 256 against 220 us (32768).
 struct BlockPack {
   int cnt;         // blocks, 0 or 1: not packed
   int a, n;        // this lane's block: first dof and size (0: none)
@@ -1482,7 +1483,6 @@ static __device__ void advance(const MjbModel& m, const MjbData& d, int w, const
 }
 
 // forward.py:165-242 — Euler with implicit joint damping unless EULERDAMP is disabled
-template <bool PACK = true>
 static __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv;
   if (m.disableflags & DSBL_EULERDAMP) {
@@ -1516,20 +1516,19 @@ static __device__ void euler(const MjbModel& m, const MjbData& d, int w, int lan
     return;
   }
   float* L = d.qLD_integration + W(w, nv * nv);
-  factor_blocks<PACK>(m, d.qM + W(w, nv * nv), L, lane, m.dof_damping, m.timestep, tile);
+  factor_blocks(m, d.qM + W(w, nv * nv), L, lane, m.dof_damping, m.timestep, tile);
   for (int i = lane; i < nv; i += 32) x[i] = sm[i] + qc[i];
   __syncwarp();
   if (m.precision && tile)  // the float factor stays in qLD_integration; x in FP64
-    factor_solve_blocks_d<PACK>(m, d.qM + W(w, nv * nv), m.dof_damping, m.timestep, x, x, lane,
+    factor_solve_blocks_d(m, d.qM + W(w, nv * nv), m.dof_damping, m.timestep, x, x, lane,
                           reinterpret_cast<double*>(tile + tile_floats(nv)));
   else
-    solve_blocks<PACK>(m, L, x, x, lane, tile, true);
+    solve_blocks(m, L, x, x, lane, tile, true);
   advance(m, d, w, x, lane);
 }
 
 // forward.py:245-405 — implicitfast (dense): (M - dt qDeriv) qacc = qfrc_smooth + qfrc_constraint
 // with qDeriv = moment^T diag(bias_vel + gain_vel * ctrl) moment - diag(damping)
-template <bool PACK = true>
 static __device__ void implicit(const MjbModel& m, const MjbData& d, int w, int lane, float* tile = nullptr) {
   const int nv = m.nv, nu = m.nu;
   const bool passive_on = !(m.disableflags & DSBL_PASSIVE);
@@ -1602,11 +1601,11 @@ static __device__ void implicit(const MjbModel& m, const MjbData& d, int w, int 
     }
   }
   if (!tiled) {
-    factor_blocks<PACK>(m, Mi, L, lane, nullptr, 0.f, tile);
-    solve_blocks<PACK>(m, L, x, f, lane);
+    factor_blocks(m, Mi, L, lane, nullptr, 0.f, tile);
+    solve_blocks(m, L, x, f, lane);
   }
   if (m.precision && tile)  // the float factor stays in qLD_integration; x again in FP64
-    factor_solve_blocks_d<PACK>(m, Mi, nullptr, 0.f, x, f, lane,
+    factor_solve_blocks_d(m, Mi, nullptr, 0.f, x, f, lane,
                           reinterpret_cast<double*>(tile + tile_floats(nv)));
   advance(m, d, w, x, lane);
 }
