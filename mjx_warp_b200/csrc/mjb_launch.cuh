@@ -68,12 +68,19 @@ int resident_ctas(K kernel, int threads, size_t smem) {
   return n;
 }
 
-// the one-warp-per-world solvers, spw floats of shared memory per warp: the chosen form's persistent
+// the Data has the arrays of k_order_worlds' schedule
+inline bool scheduled(const MjbData* d) { return d->world_order && d->work_queue && d->world_nefc; }
+
+// the one-warp-per-world solvers for nv <= 32 and a dense mass matrix, spw floats of shared memory per warp: the chosen form's persistent
 // one of FP32 FMAs at 5 CTAs per SM (mjb_solver_queue.cu); at 4, or with the Hessian on the tensor
 // pipe (mjb_solver_alt.cu); the precision form's (mjb_solver_prec.cu); the plain form's (mjb_solver_plain.cu)
 void launch_solver_warp(const MjbModel* m, const MjbData* d, int warps, int spw, cudaStream_t s);
 void launch_solver_warp_alt(const MjbModel* m, const MjbData* d, bool tc, int warps, int spw, cudaStream_t s);
 void launch_solver_warp_prec(const MjbModel* m, const MjbData* d, int warps, int spw, cudaStream_t s);
+// the generic solver for the other models, and for the worlds of more than min_rows rows
+// (mjb_solver_generic.cu)
+void launch_solver_generic(const MjbModel* m, const MjbData* d, int warps, cudaStream_t s);
+void launch_solver_many_rows(const MjbModel* m, const MjbData* d, int min_rows, cudaStream_t s);
 int launch_solver_plain(const MjbModel* m, const MjbData* d, cudaStream_t s);
 // mjb_step_fused.cu: the single form
 void launch_step_fused(const MjbModel* m, const MjbData* d, int integrate, int warps, int spw, size_t smem, cudaStream_t s);

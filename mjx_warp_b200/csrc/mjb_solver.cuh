@@ -362,9 +362,8 @@ __device__ __forceinline__ void linesearch_with(SolverCtx& s, MulM&& mulm, RowDo
   __syncwarp();
 }
 
-// solve_generic's, compiled apart: inlined into it the two held each other's registers (4096 worlds of a
-// 40-dof chain, forward 7.3 -> 7.1 ms, 2048 of a 100-dof chain 22.7 -> 21.8, the plain form's humanoid
-// 733 -> 723 us).
+// solve_generic's, compiled apart: inlined into it the two held each other's registers (forward of 2048
+// worlds of 20 boxes 11.7 -> 10.5 ms, the plain form's humanoid, 8192 worlds, 733 -> 724 us).
 static __device__ __noinline__ void linesearch(SolverCtx& s) {
   linesearch_with(s, [&]() { mul_m_ctx(s, s.mv, s.search); },
                   [&](int k) {
@@ -1143,8 +1142,8 @@ __device__ void solve_small_run(Small& s) {
 
 // solver.py:872-1000 for nv <= 32; sm: solver_smem_floats(nv) floats of warp-private scratch
 // PREC: the precision form (FP64 Hessian factor-solve and line-search sums; the double tile at
-// sm + solver_smem_floats(nv))
-template <bool PREC = false, bool TC = false>
+// sm + solver_smem_floats(nv)); ALL: CG and the parallel line search too
+template <bool PREC = false, bool TC = false, bool ALL = true>
 __device__ void solve_small(const MjbModel& m, const MjbData& d, int w, int lane, float* sm,
                             bool reuse) {
   const int nv = m.nv;
@@ -1182,7 +1181,7 @@ __device__ void solve_small(const MjbModel& m, const MjbData& d, int w, int lane
   s.gtol = 0.f;
   s.qg[0] = s.qg[1] = s.qg[2] = 0.f;
   __syncwarp();
-  const bool cg = m.solver == 1, lsp = m.ls_parallel != 0;
+  const bool cg = ALL && m.solver == 1, lsp = ALL && m.ls_parallel != 0;
   if (n <= kLaneRows) {
     if (!cg && !lsp) solve_small_run<PREC, 1, false, false, TC>(s);
     else if (!cg) solve_small_run<PREC, 1, false, true, TC>(s);

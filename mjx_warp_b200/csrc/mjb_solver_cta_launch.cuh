@@ -34,7 +34,7 @@ inline void launch_cta_form(const MjbModel* m, const MjbData* d, int tc, cudaStr
   const size_t bytes = size_t(cta_solver_smem_floats(m->nv, NW, PREC, TREES)) * sizeof(float);
   static size_t conf[kSmemDevices];
   allow_smem(k_solve_cta<NW, PREC, TREES>, bytes, conf);
-  if (d->world_order && d->work_queue && d->world_nefc) {
+  if (scheduled(d)) {
     const int ctas = resident_ctas(k_solve_cta<NW, PREC, TREES>, 32 * NW, bytes);  // ordered in phase 0
     k_solve_cta<NW, PREC, TREES><<<std::min(ctas, d->nworld), 32 * NW, bytes, s>>>(*m, *d, tc);
   } else {
