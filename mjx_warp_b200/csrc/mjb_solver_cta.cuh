@@ -338,7 +338,6 @@ struct SparseShape {
                        kNodes = kSpTrees + kPanels;  // nodes: a tree's dofs within one panel
   unsigned long long tmask[kSpTrees];      // trees u <= t with L(t, u) != 0, t itself among them
   unsigned long long tup[kSpTrees];        // trees t > u with L(t, u) != 0
-  unsigned long long cmask[kDofs / 8];   // 8-column chunks != 0 in each 8-row tile of L
   unsigned long long ptrees[kPanels];    // trees with dofs in each 32-column panel
   float cj[kJ];                          // staged row entries (tree u's, then tree t's)
   float cl[kL];                          // L, each tree's rows over its nonzero columns
@@ -364,7 +363,7 @@ struct SparseShape {
   uint8_t ntree[kNodes];                 // its tree
   uint8_t dtree[kDofs];                  // tree of each dof
   SparseOrder<kNodes> fwd, bwd;
-  int nblk, compact;
+  int nblk;
   unsigned cnt[kSpTrees];
 
   // column of tree u's first dof in tree t's rows of L
@@ -535,10 +534,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
     int f0, f1;
     const int b0 = warp_excl_scan(w0 * z0, lane, &f0), b1 = warp_excl_scan(w1 * z1, lane, &f1) + f0;
     const bool compact = f0 + f1 <= SH::kL;
-    if (lane == 0) {
-      S.L = compact ? S.cl : H;
-      S.compact = compact;
-    }
+    if (lane == 0) S.L = compact ? S.cl : H;
     S.rbase[lane] = compact ? b0 : int(S.tadr[min(lane, nt)]) * nv;
     S.rld[lane] = uint16_t(compact ? w0 : nv);
     S.rbase[lane + 32] = compact ? b1 : int(S.tadr[min(lane + 32, nt)]) * nv;
@@ -567,20 +563,7 @@ __device__ __noinline__ bool sparse_shape(const MjbModel& m, const float* J, int
       e += __popc(mk);
     }
   }
-  const int n8 = (nv + 7) >> 3, n32 = (nv + 31) >> 5;
-#pragma unroll 1
-  for (int r = tid; r < n8; r += NT) {  // 8-row tiles: the chunks of their rows' trees
-    const int t0 = S.dtree[8 * r], t1 = S.dtree[min(8 * r + 7, nv - 1)];
-    unsigned long long tm = 0ull, cm = 0ull;
-#pragma unroll 1
-    for (int t = t0; t <= t1; t++) tm |= S.tmask[t];
-#pragma unroll 1
-    for (; tm; tm &= tm - 1ull) {
-      const int u = __ffsll(tm) - 1;
-      cm |= bits_below(((S.tadr[u + 1] - 1) >> 3) + 1) & ~bits_below(S.tadr[u] >> 3);
-    }
-    S.cmask[r] = cm & bits_below(r + 1);
-  }
+  const int n32 = (nv + 31) >> 5;
 #pragma unroll 1
   for (int p = warp; p < n32; p += NW) {
     const int c0 = 32 * p, c1 = min(c0 + 32, nv), pn = c1 - c0;
