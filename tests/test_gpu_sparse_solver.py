@@ -9,7 +9,8 @@ import pytest
 import torch
 
 import mjx_warp_b200 as mjw
-from mjx_warp_b200.types import MJ_JAC_DENSE
+from mjx_warp_b200.types import MJ_JAC_DENSE, MJ_JAC_SPARSE
+from oracle import Oracle
 from helpers import dev, device_data, load, world_rows
 from test_gpu_configs import bin_state, humanoid_spheres_state
 
@@ -34,6 +35,21 @@ def chain_xml(n):
   return s + "</body>" * n + "</worldbody></mujoco>"
 
 
+def star_xml(n, dofs):
+  """n trees resting on one long capsule, the first tree, whose elimination couples them all: free
+  capsules, each with dofs - 6 hinges hanging from it."""
+  s = ('<mujoco><option timestep="0.002"/><worldbody><body pos="0 0 1"><freejoint/>'
+       f'<geom type="capsule" fromto="0 0 0 {0.5 * n:g} 0 0" size="0.1"/></body>')
+  for i in range(n):
+    s += (f'<body pos="{0.25 + 0.5 * i} 0 1.19"><freejoint/>'
+          '<geom type="capsule" fromto="0 -0.1 0 0 0.1 0" size="0.1"/>')
+    for k in range(dofs - 6):
+      s += (f'<body pos="0 0 0.05"><joint type="hinge" damping="0.3" axis="{k % 2} {(k + 1) % 2} 0.2"/>'
+            '<geom type="capsule" fromto="0 0 0 0 0 0.05" size="0.02" contype="0" conaffinity="0"/>')
+    s += "</body>" * (dofs - 5)
+  return s + "</worldbody></mujoco>"
+
+
 def case(name):
   """(model, qpos, qvel, ctrl, rows capacity per world)"""
   opt = dict(iterations=0, ls_iterations=10, jacobian=MJ_JAC_DENSE)
@@ -45,6 +61,12 @@ def case(name):
     x[:, :, :2] += rng.uniform(-0.12, 0.12, x[:, :, :2].shape)
     x[0, :, 2] += 5.0  # a world without rows
     return mjm, q, rng.normal(0.0, 0.1, (5, mjm.nv)), np.zeros((5, 0)), 512
+  if name.startswith("star"):
+    mjm = load(star_xml(*(int(n) for n in name[4:].split("x"))), **opt)
+    rng = np.random.default_rng(8)
+    q = np.tile(mjm.qpos0, (3, 1))
+    q[1, 2] -= 0.5  # a world whose trees do not touch
+    return mjm, q, rng.normal(0.0, 0.01, (3, mjm.nv)), np.zeros((3, 0)), 256
   if name == "humanoid_spheres":
     mjm = load("humanoid_spheres.xml", **opt)
     q, v, u, _ = humanoid_spheres_state(mjm, load("humanoid.xml"), 8, seed=3)
@@ -76,9 +98,10 @@ def tree_pairs(mjm, J):
 
 @pytest.mark.parametrize("warps", [2, 4])
 @pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres64", "spheres65", "humanoid_spheres",
-                                  "bin", "bin_rows", "bin_pairs"])
+                                  "bin", "bin_rows", "bin_pairs", "star20x22", "star29x17"])
 def test_factor_of_the_hessian(name, warps):
-  """With no iterations efc_h is the factor of H = qM + J_a' D_a J_a at the warmstart's active set:
+  """Also past the lists of a panel's updated tiles (20 coupled trees of 22 dofs) and of its rows below (29 of
+  17), with few rows.  With no iterations efc_h is the factor of H = qM + J_a' D_a J_a at the warmstart's active set:
   zero where H's factor is, and L L' = H within the backward error of an FP32 Cholesky factorisation
   (nv + 1 roundings of 2^-24 per entry, doubled for the assembly)."""
   mjm, q, v, u, cap = case(name)
@@ -112,11 +135,11 @@ def test_factor_of_the_hessian(name, warps):
     assert r < 2 * (mjm.nv + 1) * 2.0 ** -24, (w, r)
 
 
-@pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres16", "humanoid_spheres"])
+@pytest.mark.parametrize("name", ["spheres6", "spheres11", "spheres16", "humanoid_spheres", "star18x6"])
 def test_one_warp_form_equals_plain(name):
   """Up to 128 dofs the chosen form solves a world by one warp over the nonzero trees in the plain
   form's arithmetic: equal values, whether the world fits the structure or (more than 192 rows: the
-  16 spheres in one heap) takes the generic solver."""
+  16 spheres in one heap; more than 160 tree pairs: 18 capsules on one) takes the generic solver."""
   mjm, q, v, u, cap = case(name)
   mjm.opt.iterations = 10
   if name == "spheres16":
@@ -133,6 +156,10 @@ def test_one_warp_form_equals_plain(name):
     out[form] = d
   n = world_rows(out[1], "efc")[0]
   assert name != "spheres16" or n.max() > 192 > n.min()
+  if name == "star18x6":
+    idx = world_rows(out[1], "efc")[1]
+    J = out[1].efc.J.cpu().numpy()
+    assert n[0] <= 192 and tree_pairs(mjm, J[idx[:n[0]]]) > 160
   for f in ("qacc", "qfrc_constraint"):
     assert torch.equal(getattr(out[1], f), getattr(out[0], f)), f
   for f in ("cost", "Ma", "h"):
@@ -247,3 +274,30 @@ def test_nonfinite_force_reaches_every_tree(name, bad):
   assert not plain[1].any() and np.delete(plain, 1, axis=0).all()
   assert np.array_equal(np.isfinite(qacc["chosen"]), plain)
   assert np.array_equal(np.delete(qacc["chosen"], 1, axis=0), np.delete(qacc["clean"], 1, axis=0))
+
+
+@pytest.mark.parametrize("jacobian", [MJ_JAC_DENSE, MJ_JAC_SPARSE])
+@pytest.mark.parametrize("solver, iterations, ls_iterations, ls_parallel",
+                         [(2, 20, 20, False), (2, 20, 50, True), (1, 100, 20, False), (1, 100, 50, True)])
+@pytest.mark.parametrize("name", ["spheres11", "humanoid_spheres", "bin"])
+def test_solvers_and_searches_over_trees(name, solver, iterations, ls_iterations, ls_parallel, jacobian):
+  """Newton and CG, the iterative and the parallel search, dense and sparse mass matrix, one warp (66 and 123
+  dofs) and four warps (384): the cost is the oracle's, by the reference's acceptance (solver_test.py:
+  2.5 % above it at most)."""
+  mjm, q, v, u, cap = case(name)
+  mjm.opt.solver, mjm.opt.iterations, mjm.opt.ls_iterations, mjm.opt.jacobian = solver, iterations, ls_iterations, jacobian
+  nworld = q.shape[0]
+  m = mjw.put_model(mjm)
+  m.opt.ls_parallel = ls_parallel
+  d = device_data(mjm, q, v, u, nconmax=800 * nworld, njmax=cap * nworld)
+  mjw.forward(m, d)
+  torch.cuda.synchronize()
+  assert m.opt.is_sparse == (jacobian == MJ_JAC_SPARSE) and np.all(mjw.world_status(d) == 0)
+  o = Oracle(mjm, nworld, 64, ls_parallel=ls_parallel)
+  for f, x in (("qpos", q), ("qvel", v), ("ctrl", u)):
+    if x.shape[1]:
+      o.set(f, x)
+  o.run("forward", nthreads=8)
+  np.testing.assert_array_equal(world_rows(d, "efc")[0], o.rows("efc_D")[0])
+  cost, ref = d.efc.cost.cpu().numpy(), o.scalar("cost")
+  assert np.all(cost <= ref + 0.025 * np.abs(ref) + 1e-3), (cost, ref)
