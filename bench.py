@@ -176,6 +176,28 @@ def _solver_flops(nv, rows, iters, ls_iters):
   return (1 + iters) * (f_h + f_chol) + iters * (4.0 * nv * nv + 4.0 * rows * nv + 24.0 * ls_iters * rows)
 
 
+def _tree_solver_flops(mjm, J, iters, ls_iters):
+  """_solver_flops of one world over what is not exactly zero, for a model of many kinematic trees: row r of
+  J (rows x nv) touches t_r dofs, and column k of the factor of H has c_k nonzeros below the diagonal (the
+  tree pairs that the rows couple and the fill of eliminating the trees in dof order):
+  F_H = sum t_r (t_r + 1), F_chol = sum c_k (c_k + 1) + 4 (nv + sum c_k), F_Mv = 2 sum over trees of their
+  dofs squared, F_Jv = 2 sum t_r, F_ls = 24 L R."""
+  tree = np.unique(np.asarray(mjm.body_rootid)[np.asarray(mjm.dof_bodyid)], return_inverse=True)[1]
+  n, size = tree.max() + 1, np.bincount(tree)
+  t = np.count_nonzero(J, axis=1).astype(float)
+  touch = np.stack([np.any(J[:, tree == k] != 0, axis=1) for k in range(n)], axis=1).astype(int)
+  C = (touch.T @ touch > 0) | np.eye(n, dtype=bool)
+  for k in range(n):
+    later = np.nonzero(C[k + 1:, k])[0] + k + 1
+    C[np.ix_(later, later)] = True
+  below = np.tril(C, -1).astype(float).T @ size  # dofs of the later trees coupled with each tree
+  c = np.concatenate([below[k] + np.arange(size[k])[::-1] for k in range(n)])
+  f_chol = np.sum(c * (c + 1.0)) + 4.0 * (len(c) + np.sum(c))
+  f_mv, f_jv = 2.0 * np.sum(size.astype(float) ** 2), 2.0 * np.sum(t)
+  return ((1 + iters) * (np.sum(t * (t + 1.0)) + f_chol)
+          + iters * (2.0 * f_mv + 2.0 * f_jv + 24.0 * ls_iters * len(J)))
+
+
 def _step_flops(mjm, rows, pairs, contacts):
   """Algorithmic flops of one world-step: smooth dynamics (~600 per body, 60 per geom), collision
   (20 per broadphase pair, 150 per contact), constraint assembly (R (6 nv + 40)), the mass-matrix
@@ -534,9 +556,12 @@ def _bin_config(mjw, torch, nworld=4096, steps=500, plain_steps=10, sample=16):
   solve_s = a.elapsed_time(b) * 1e-3
   rows_solve = int(d.world_nefc.sum()) / nworld
   fma = _fma_peaks(torch)
-  flops = _solver_flops(mjm.nv, rows_solve, mjm.opt.iterations, mjm.opt.ls_iterations) * nworld
   # qacc of one forward from the final state against FP64 on a sample
   s = min(sample, nworld)
+  adr, cnt = (x[:s].cpu().numpy() for x in (d.world_efcadr, d.world_nefc))
+  flops = nworld * float(np.mean([_tree_solver_flops(mjm, d.efc.J[a:a + n].cpu().numpy(),
+                                                     mjm.opt.iterations, mjm.opt.ls_iterations)
+                                  for a, n in zip(adr, cnt)]))
   host = {k: getattr(d, k)[:s].double().cpu().numpy() for k in ("qpos", "qvel", "qacc_warmstart")}
   mjw.forward(m, d)
   qd = d.qacc[:s].double().cpu().numpy()
@@ -576,7 +601,7 @@ def _bin_config(mjw, torch, nworld=4096, steps=500, plain_steps=10, sample=16):
                        "flops_per_launch": flops, "achieved_tflops": flops / solve_s / 1e12,
                        "peak_tflops": fma["fp32_tflops"],
                        "frac": flops / solve_s / 1e12 / fma["fp32_tflops"], "bound": "fp32",
-                       "rows_per_world": rows_solve}}
+                       "flops_counted": f"nonzero tree pairs of {s} worlds", "rows_per_world": rows_solve}}
 
 
 def _profile_case_bin(mjw, torch, nworld=512, cta_warps=2):
