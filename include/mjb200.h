@@ -237,7 +237,7 @@ typedef struct MjbTune {
   int32_t solver_cta_warps;  /* 2, 4, 8 or 16 warps per world; 0 = one warp per world */
   int32_t hessian_tc;        /* nv <= 32: 1 = Newton Hessian in split TF32 on the tensor pipe */
   int32_t solver_ctas_per_sm; /* nv <= 32, FMA Hessian: resident CTAs per SM of the persistent
-                                 solver, 4 (128 registers) or 5 (96); 0 in mjb_set_tune = 5 */
+                                 solver, 4 (128 registers) or 5 (96); 0 in mjb_set_tune = 4 */
   float ms_per_forward;      /* measured chosen-form forward (fwd_position .. solve) at this setting */
   float rows_per_world;      /* mean constraint rows per world of the Data it was measured on */
 } MjbTune;

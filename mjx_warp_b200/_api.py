@@ -332,7 +332,7 @@ def set_tune(m: Model, d: Data, tree_lanes: int = 16, solver_warps: int = 4,
   autotune): lanes per world of the tree-recursion stages (8, 16, 32), warps per CTA of the
   one-warp-per-world solver (1, 2, 4), its Newton Hessian on the tensor pipe in split TF32
   (hessian_tc, nv <= 32), its resident CTAs per SM with the FMA Hessian (solver_ctas_per_sm: 4
-  or 5, 0 for the default 5) and warps per world of the CTA solver of models with nv > 32
+  or 5, 0 for the default 4) and warps per world of the CTA solver of models with nv > 32
   (2, 4, 8, 16, or 0 for one warp per world)."""
   t = _abi.MjbTune()
   t.tree_lanes, t.solver_warps, t.solver_cta_warps = tree_lanes, solver_warps, solver_cta_warps

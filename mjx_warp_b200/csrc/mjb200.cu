@@ -550,7 +550,7 @@ struct ChosenCfg {
   int warps = kDefaultWarps;
   int cta_warps = 4;  // warps per world of the solver for nv > 32 (0: one warp per world)
   int hessian_tc = 0; // nv <= 32: Newton Hessian on the tensor pipe (split TF32) instead of FMAs
-  int solver_ctas = 5;  // CTAs per SM of the FP32 FMA-Hessian persistent solver (4, 5)
+  int solver_ctas = 4;  // CTAs per SM of the FP32 FMA-Hessian persistent solver (4, 5)
 };
 struct TuneEntry {
   int dev, nv, cap;

@@ -72,8 +72,8 @@ int resident_ctas(K kernel, int threads, size_t smem) {
 inline bool scheduled(const MjbData* d) { return d->world_order && d->work_queue && d->world_nefc; }
 
 // the one-warp-per-world solvers for nv <= 32 and a dense mass matrix, spw floats of shared memory per warp: the chosen form's persistent
-// one of FP32 FMAs at 5 CTAs per SM (mjb_solver_queue.cu); at 4, or with the Hessian on the tensor
-// pipe (mjb_solver_alt.cu); the precision form's (mjb_solver_prec.cu); the plain form's (mjb_solver_plain.cu)
+// one of FP32 FMAs at 5 CTAs per SM (mjb_solver_queue.cu); at 4, the default, or with the Hessian on the
+// tensor pipe (mjb_solver_alt.cu); the precision form's (mjb_solver_prec.cu); the plain form's (mjb_solver_plain.cu)
 void launch_solver_warp(const MjbModel* m, const MjbData* d, int warps, int spw, cudaStream_t s);
 void launch_solver_warp_alt(const MjbModel* m, const MjbData* d, bool tc, int warps, int spw, cudaStream_t s);
 void launch_solver_warp_prec(const MjbModel* m, const MjbData* d, int warps, int spw, cudaStream_t s);
