@@ -715,7 +715,7 @@ void launch_solver(const MjbModel* m, const MjbData* d, const ChosenCfg& cfg, in
     }
   }
   if (PREC) launch_solver_warp_prec(m, d, cfg.warps, spw, s);
-  else if (m->nv > 32 || m->is_sparse) launch_solver_generic(m, d, cfg.warps, s);
+  else if (!small_model(*m)) launch_solver_generic(m, d, cfg.warps, s);
   else if (cfg.hessian_tc || cfg.solver_ctas == 4) launch_solver_warp_alt(m, d, cfg.hessian_tc != 0, cfg.warps, spw, s);
   else launch_solver_warp(m, d, cfg.warps, spw, s);
 }

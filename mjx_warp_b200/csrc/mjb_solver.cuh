@@ -1202,17 +1202,8 @@ __device__ void solve_small(const MjbModel& m, const MjbData& d, int w, int lane
   }
 }
 
-// Dispatch: the register / shared-memory solver when nv <= 32 and the caller provides its scratch
-// (solver_smem_floats(nv) floats), else the generic solver with an nv x nv Hessian tile `hs`.
-// reuse: keep the Newton Hessian's factor across iterations with an unchanged active set.
-// For nv > 32 or a sparse mass matrix, sm (when given) is the generic solver's scratch of at least
-// generic_nz_floats(nv) floats.
-// TC: the Newton Hessian of staged rows assembled on the tensor pipe (split TF32, hessian_tc)
-template <bool PREC = false, bool TC = false>
-__device__ __forceinline__ void solve(const MjbModel& m, const MjbData& d, int w, int lane,
-                                      float* sm, float* hs, bool reuse = false) {
-  if (m.nv <= 32 && sm && !m.is_sparse) solve_small<PREC, TC>(m, d, w, lane, sm, reuse);
-  else solve_generic(m, d, w, lane, hs, (m.nv > 32 || m.is_sparse) ? sm : nullptr, reuse);
-}
+// The host launches solve_small's kernels for nv <= 32 with a dense mass matrix, solve_generic's for the
+// rest (nz: the warp's scratch of at least generic_nz_floats(nv) floats, 2 round4(nv) for nv <= 32).
+inline bool small_model(const MjbModel& m) { return m.nv <= 32 && !m.is_sparse; }
 
 }  // namespace mjb
