@@ -692,8 +692,9 @@ int run_forward_plain(const MjbModel* m, const MjbData* d, cudaStream_t s) {
   return d->njmax == 0 ? MJB_OK : launch_stage<S_SOLVE>(m, d, s);
 }
 
-// the chosen form's solver launch: k_order_worlds + the persistent k_solve_queue when the Data has
-// the schedule arrays, else one warp per world (k_solve); PREC selects the precision form's solver
+// the chosen form's solver launch (mjb_launch.cuh): persistent kernels over k_order_worlds' order when the
+// Data has the schedule arrays, else one warp or CTA per world in index order; PREC selects the
+// precision form's solver
 template <bool PREC>
 void launch_solver(const MjbModel* m, const MjbData* d, const ChosenCfg& cfg, int spw,
                    cudaStream_t s) {
